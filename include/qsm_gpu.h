@@ -275,8 +275,9 @@ typedef struct {
     double seconds;         /* device time */
     double *resnorm_hist;   /* optional, caller-owned, >= maxitcg doubles */
     int32_t coarse_ctas;    /* coarsest-level solver: 0 host-driven loop, 1 one CTA,
-                               > 1 a thread-block cluster of that many CTAs, < 0 a
-                               cooperative launch of -coarse_ctas CTAs (one per SM) */
+                               > 1 a thread-block cluster of that many CTAs, < 0
+                               (passes of more than 6000 voxels) -coarse_ctas CTAs, one
+                               per SM: a cooperative launch in FP64, a cluster in FP32 */
     int32_t coarse_outer;   /* outer iterations (256 sweeps each) it ran in total */
 } qsm_mg_info;
 

@@ -18,10 +18,12 @@
 //                           public gauss_seidel_mex and grids without lists
 //   coarsest level          the reference's <= 1024 x (128 reverse + 128
 //                           forward sweeps + residual + norm) loop in one
-//                           launch: z-slabs over a 16-CTA cluster in shared
-//                           memory (small grids), over every SM with a grid
-//                           barrier (large passes), or in one CTA; the norm
-//                           keeps the lane order; no host round trips
+//                           launch: in chunks over a cluster of 1 or 16 CTAs
+//                           (mg_slab.cuh: FP32, and small FP64 grids), over
+//                           every SM with a grid barrier (large FP64 passes),
+//                           in z-slabs or on one CTA (grids without voxel
+//                           lists, packed solves); the norm keeps the lane
+//                           order; no host round trips
 //   PCG                     the BLAS-1 steps fused into four kernels on the
 //                           lane-dot grid; scalars stay on the device and the
 //                           host reads ||r|| once per iteration; where the
@@ -1457,6 +1459,8 @@ __global__ void __launch_bounds__(CC_THREADS) coarse_cluster_k(T *gv, const T *_
     cl_sync();  // no CTA leaves while a peer may still address its shared memory
 }
 
+#include "mg_slab.cuh"
+
 // ---------------------------------------------------------------------------
 // hierarchy and drivers (mgpcg_mex.c:126-332, mg_mex.c:94-207, fmg_mex.c:93-212)
 // ---------------------------------------------------------------------------
@@ -1501,6 +1505,8 @@ struct Hier {
     int cc_ctas;         // > 0: the coarsest level runs on a cluster of this many CTAs
     int cc_npmax;        // planes per CTA (largest slab)
     size_t cc_smem;
+    SlabTab sl;          // sl.ctas > 0: the coarsest level runs in chunks on a cluster of that many CTAs
+    bool sl_large;       // its colour passes are those the whole GPU would take in FP64
 };
 
 static inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -1703,6 +1709,113 @@ static void plan_coarse_grid(qsm_ctx *ctx, Hier<T> &H)
     H.cg_ctas = sms;
 }
 
+// The slab solver's kernel for a plan's voxels per thread.
+template <typename T>
+static const void *slab_kernel(int per)
+{
+    return per == 1 ? (const void *)coarse_slab_k<T, 1> : (const void *)coarse_slab_k<T, SL_MAX_PER>;
+}
+
+// The slab solver's dynamic shared-memory limit (as cluster_smem_limit).
+template <typename T>
+static size_t slab_smem_limit(qsm_ctx *ctx)
+{
+    static std::mutex mu;
+    static size_t lim[64];
+    static bool done[64];
+    std::lock_guard<std::mutex> lock(mu);
+    const int dv = ctx->device & 63;
+    if (done[dv]) return lim[dv];
+    done[dv] = true;
+    int maxsm = 0;
+    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    size_t l = (size_t)-1;
+    for (int per = 1; per <= SL_MAX_PER; per += SL_MAX_PER - 1) {
+        cudaFuncAttributes fa;
+        const void *k = slab_kernel<T>(per);
+        if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || (size_t)maxsm <= fa.sharedSizeBytes ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)((size_t)maxsm - fa.sharedSizeBytes)) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        l = std::min(l, (size_t)maxsm - fa.sharedSizeBytes);
+    }
+    return lim[dv] = l;
+}
+
+template <typename T>
+static cudaLaunchConfig_t slab_config(const SlabTab &t, cudaLaunchAttribute *at)
+{
+    cudaLaunchConfig_t cfg = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)t.ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)t.ctas);
+    cfg.blockDim = dim3((unsigned)t.threads);
+    cfg.dynamicSmemBytes = t.smem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// CTAs of the slab solver for c0 and c1 coarsest G voxels of the colours (0:
+// another solver's).  Whole FP32 / FP64 solves in ms, this solver against the
+// one it takes over from (LBV options, 8-10 PCG iterations, ~20-80 calls of
+// 512 passes each; voxels per colour in brackets):
+//   FP32, up to 1024: one CTA 15.0 against 15.4 (256^3 [640]), 4.3 against 4.6
+//     (64^3), 4.8 against 5.3 (80^2 x 60); 16 CTAs would take 17.1, 6.0, 6.3
+//   FP32, above: 16 CTAs 11.4 against 12.6 on the z-slab cluster (181 x 217 x
+//     155 [2k]), 9.1 against 12.5 (150 x 120 x 100 [4.4k]); 13.6 against 41.7
+//     and 6.9 against 26.9 over the whole GPU (190^2 x 110 [11k], 96 x 100 x 40)
+//   FP64, up to CG_MIN_PASS: 16 CTAs 36.8 against 37.6 (256^3), 27.1 against
+//     41.0 (181 x 217 x 155), 32.5 against 62.3 (150 x 120 x 100).
+// Longer FP64 passes are bound by 16 SMs' FP64 pipes.
+template <typename T>
+static int slab_ctas(unsigned c0, unsigned c1)
+{
+    const unsigned c = std::max(c0, c1);
+    if (sizeof(T) == 4) return c <= 1024u ? 1 : SL_MAX_CTAS;
+    return c <= CG_MIN_PASS ? SL_MAX_CTAS : 0;
+}
+
+// Plans the slab solver of the coarsest level (c0, c1: its G voxels of each
+// colour, cut: its chunks); returns the bytes of its table, 0 where another
+// solver runs.
+template <typename T>
+static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, const unsigned *cut)
+{
+    const Level<T> &C = H.L[H.nl - 1];
+    SlabTab &t = H.sl;
+    t.ctas = 0;
+    if (C.d.nx < 3 || C.d.ny < 3 || C.d.nz < 3 || C.n > RED_LANES) return 0;
+    const int ctas = slab_ctas<T>(c0, c1);
+    const size_t lim = slab_smem_limit<T>(ctx);
+    if (ctas <= 0 || lim == 0) return 0;
+    t.cap = 1;
+    for (int c = 0, st = SL_MAX_CTAS / ctas; c < SL_MAX_CTAS; c += st)
+        for (int q = 0; q < 2; ++q) t.cap = std::max(t.cap, cut[2 * (c + st) + q] - cut[2 * c + q]);
+    t.win = ctas > 1 ? (unsigned)((C.d.ny + 1) * ((C.d.nx - 1) / 2) + 2) : 0u;
+    t.per = t.cap <= (unsigned)SL_MAX_THREADS ? 1 : SL_MAX_PER;
+    t.threads = std::max(64, (int)(((t.cap + t.per - 1) / t.per + 31) / 32 * 32));
+    const SlabLayout lay(t.cap, t.win, ctas, sizeof(T));
+    t.smem = lay.bytes;
+    if (t.threads > SL_MAX_THREADS || lay.bytes > lim || lay.len > 0xFFFFu) return 0;
+    t.ctas = ctas;
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = slab_config<T>(t, at);
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, slab_kernel<T>(t.per), &cfg) != cudaSuccess || ncl < 1) {
+        cudaGetLastError();
+        t.ctas = 0;
+        return 0;
+    }
+    H.sl_large = c0 > CG_MIN_PASS || c1 > CG_MIN_PASS;
+    return al256(C.n * sizeof(unsigned));
+}
+
 // Colour lists of every level's G and boundary band B (counted, then filled
 // into one allocation), and how each list's passes run (by its size).
 // Grids of 2^30 voxels or more keep the full-grid passes.
@@ -1712,7 +1825,8 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
     if (H.L[0].n >= ((size_t)1 << 30)) return QSM_OK;
     const int cn = sweeps_cluster_size<T>(ctx);
     unsigned *cnt = (unsigned *)H.counters + 8;  // B: 4i, 4i+1; G: 4i+2, 4i+3 (nl <= 16)
-    QSM_CUDA(cudaMemsetAsync(cnt, 0, 4 * H.nl * sizeof(unsigned), ctx->stream));
+    const int ncnt = 4 * H.nl + 2 * (SL_MAX_CTAS + 1);  // then the coarsest level's cuts
+    QSM_CUDA(cudaMemsetAsync(cnt, 0, ncnt * sizeof(unsigned), ctx->stream));
     // per level: segment counts of its four lists (B and G, two colours each) and their scan
     size_t nseg[16] = {0}, tot_seg = 0, max_seg = 0;
     for (int i = 0; i < H.nl; ++i) {
@@ -1733,10 +1847,12 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
         QSM_CUDA(cudaGetLastError());
         QSM_TRY(exclusive_scan(ctx, segc + o, segoff + o, 4 * nseg[i], scan_tmp));
         blist_total_k<<<1, 32, 0, ctx->stream>>>(segc + o, segoff + o, nseg[i], cnt + 4 * i);
+        if (i + 1 == (size_t)H.nl)
+            slab_cuts_k<<<1, 32, 0, ctx->stream>>>(cnt + 4 * H.nl, segoff + o, cnt + 4 * i, (unsigned)nseg[i]);
     }
     QSM_CUDA(cudaGetLastError());
-    unsigned hc[64];
-    QSM_CUDA(cudaMemcpyAsync(hc, cnt, 4 * H.nl * sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    unsigned hc[64 + 2 * (SL_MAX_CTAS + 1)];
+    QSM_CUDA(cudaMemcpyAsync(hc, cnt, ncnt * sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     QSM_CUDA(cudaStreamSynchronize(ctx->stream));
     size_t tot = 0;
     H.sg_ctas = grid_sweep_ctas<T>(ctx);
@@ -1755,7 +1871,8 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
         for (int p = 0; p < 2; ++p)
             tot += al256((size_t)hc[4 * i + p] * sizeof(uint32_t)) + al256((size_t)hc[4 * i + 2 + p] * sizeof(uint32_t));
     }
-    QSM_TRY(dalloc(ctx, &H.lists, tot + 256));
+    const size_t sl_bytes = plan_slab<T>(ctx, H, hc[4 * (H.nl - 1) + 2], hc[4 * (H.nl - 1) + 3], hc + 4 * H.nl);
+    QSM_TRY(dalloc(ctx, &H.lists, tot + 256 + sl_bytes));
     H.sw_ctas = cn;
     char *c = (char *)H.lists;
     for (int i = 0; i < H.nl; ++i) {
@@ -1780,6 +1897,16 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
     }
     QSM_CUDA(cudaGetLastError());
     QSM_TRY(dfree(ctx, segblk));
+    if (H.sl.ctas > 0) {
+        const Level<T> &C = H.L[H.nl - 1];
+        const unsigned n01 = C.gn[0] + C.gn[1];
+        H.sl.pos = (unsigned *)c;
+        H.sl.cut = cnt + 4 * H.nl;
+        QSM_CUDA(cudaMemsetAsync(H.sl.pos, 0xFF, C.n * sizeof(unsigned), ctx->stream));
+        if (n01) slab_pos_k<<<(n01 + 255) / 256, 256, 0, ctx->stream>>>(H.sl.pos, C.gl[0], C.gn[0], C.gl[1], C.gn[1]);
+        QSM_CUDA(cudaGetLastError());
+        return QSM_OK;
+    }
     plan_coarse_grid<T>(ctx, H);
     return QSM_OK;
 }
@@ -2092,6 +2219,22 @@ static qsm_status coarse_solve(qsm_ctx *ctx, Hier<T> &H, int l, double *scal_dev
 {
     Level<T> &L = H.L[l];
     const double tol = sizeof(T) == 4 ? 1e-4 : 1e-8;
+    if (H.sl.ctas > 0) {
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = slab_config<T>(H.sl, at);
+        cfg.stream = ctx->stream;
+        T *vv = L.v, *rr = L.r;
+        const T *ff = L.f;
+        const uint32_t *la = L.gl[0], *lb = L.gl[1];
+        Dims dd = L.d;
+        GsC<T> gc = gs_consts<T>(L.h);
+        LapC<T> lc = lap_consts<T>(L.h);
+        double tl = tol;
+        int *err = H.gb.err, *outer = H.counters;
+        void *args[] = {&vv, &ff, &rr, &la, &lb, &H.sl, &dd, &gc, &lc, &tl, &err, &outer};
+        QSM_CUDA(cudaLaunchKernelExC(&cfg, slab_kernel<T>(H.sl.per), args));
+        return QSM_OK;
+    }
     if (H.cg_ctas > 0) {
         T *vv = L.v, *rr = L.r, *part = (T *)H.gpart;
         const T *ff = L.f;
@@ -2663,18 +2806,18 @@ __global__ void __launch_bounds__(RED_BLOCK) pcg_xr_k(TP *__restrict__ x, const 
 template <typename T>
 static qsm_status coarse_report(qsm_ctx *ctx, const Hier<T> &H, qsm_mg_info *info)
 {
-    if (H.cg_ctas > 0 || H.sg_ctas > 0) {
+    if (H.cg_ctas > 0 || H.sg_ctas > 0 || H.sl.ctas > 0) {
         int err = 0;
         QSM_CUDA(cudaMemcpy(&err, H.gb.err, sizeof(int), cudaMemcpyDeviceToHost));
         if (err) {
-            set_error(ctx, "multigrid: a grid barrier timed out");
+            set_error(ctx, "multigrid: a device wait timed out");
             return QSM_ERR_TIMEOUT;
         }
     }
     if (!info) return QSM_OK;
     int dev_outer = 0;
     QSM_CUDA(cudaMemcpy(&dev_outer, H.counters, sizeof(int), cudaMemcpyDeviceToHost));
-    info->coarse_ctas = H.cg_ctas > 0 ? -H.cg_ctas : H.cc_ctas > 0 ? H.cc_ctas : (H.coarse_in_smem ? 1 : 0);
+    info->coarse_ctas = H.sl.ctas > 0 ? (H.sl_large ? -H.sl.ctas : H.sl.ctas) : H.cg_ctas > 0 ? -H.cg_ctas : H.cc_ctas > 0 ? H.cc_ctas : (H.coarse_in_smem ? 1 : 0);
     info->coarse_outer = dev_outer + H.host_outer;
     return QSM_OK;
 }
@@ -3393,6 +3536,7 @@ static qsm_status mgpcg_batch_t(qsm_ctx *ctx, uint32_t count, const Dims *d, con
                 // the one-CTA form reports its coarsest solver as such
                 S.H.cc_ctas = 0;
                 S.H.cg_ctas = 0;
+                S.H.sl.ctas = 0;
                 pack.push_back(&S);
                 continue;
             }
@@ -3454,11 +3598,11 @@ qsm_status mgpack_setup(qsm_ctx *ctx, bool mixed, const Dims &d, const double *v
     if (mixed) {
         st = pcg_setup(ctx, p->sm, d, v0, f, mask, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, npost, nb, nl);
         if (st == QSM_OK) p->packable = pcg_packable(ctx, p->sm);
-        if (p->packable) p->sm.H.cc_ctas = p->sm.H.cg_ctas = 0;
+        if (p->packable) p->sm.H.cc_ctas = p->sm.H.cg_ctas = p->sm.H.sl.ctas = 0;
     } else {
         st = pcg_setup(ctx, p->sd, d, v0, f, mask, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, npost, nb, nl);
         if (st == QSM_OK) p->packable = pcg_packable(ctx, p->sd);
-        if (p->packable) p->sd.H.cc_ctas = p->sd.H.cg_ctas = 0;
+        if (p->packable) p->sd.H.cc_ctas = p->sd.H.cg_ctas = p->sd.H.sl.ctas = 0;
     }
     if (st != QSM_OK) {
         if (p->sm.pv) pcg_finish(ctx, p->sm, (double *)nullptr, (qsm_mg_info *)nullptr);

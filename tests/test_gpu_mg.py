@@ -386,3 +386,42 @@ def test_mgpcg_batch_tiny_grids_vs_oracle(gpu_ctx, qsm, port, dt_mixed):
         else:
             ref = port.mgpcg_mex(np.zeros_like(f, order="F"), f, m, *args)
         assert bits_equal(out, ref), (f.shape, first_diff(out, ref))
+
+
+@pytest.mark.parametrize("dt", ("float64", "float32"))
+@pytest.mark.parametrize("shape,nl,kind", [((30, 28, 26), 1, "ball"), ((31, 27, 26), 1, "ball"), ((30, 28, 26), 1, "v0"),
+                                           ((24, 22, 20), 1, "plates"), ((17, 19, 40), 1, "rods"), ((12, 13, 11), 1, "dots"),
+                                           ((66, 60, 52), 2, "ball"), ((58, 64, 50), 2, "box")])
+def test_coarse_chunks_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl, kind):
+    """The coarsest solver's chunks (equal shares of the G voxels in index order,
+    on 1 or 16 CTAs that send each other the values they read): masks whose
+    chunks hold part of a row, whole planes or nothing, single-voxel
+    neighbourhoods, voxels on the box's x faces (the quirk columns), both
+    parities of nx (which colour the reverse sweeps begin with), and an initial
+    guess outside the mask, which the passes read and never change.
+    Bit-for-bit against the oracle, whose arithmetic it repeats."""
+    rng = np.random.default_rng(sum(shape))
+    i, j, k = np.ogrid[0:shape[0], 0:shape[1], 0:shape[2]]
+    if kind in ("ball", "v0"):
+        m = sum(((a - (n - 1) / 2) / (0.48 * n)) ** 2 for a, n in zip((i, j, k), shape)) <= 1.0
+    elif kind == "plates":
+        m = (k % 5 == 2) & (i >= 0) & (j > 1)
+    elif kind == "rods":
+        m = ((i % 3 == 1) & (j % 4 != 0)) & (k >= 0)
+    elif kind == "dots":
+        m = rng.random(shape) < 0.35
+    else:
+        m = np.ones(shape, bool)
+    m = np.asfortranarray(np.broadcast_to(m, shape).astype(np.uint8))
+    f = np.asfortranarray((rng.standard_normal(shape) * m).astype(dt))
+    v0 = np.zeros(shape, order="F", dtype=dt)
+    if kind == "v0":
+        v0 = np.asfortranarray((0.1 * rng.standard_normal(shape)).astype(dt))
+    h = [1, 0.9, 1.2]
+    gi = {}
+    a = qsm.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl, info=gi)
+    assert gi["coarse_ctas"] != 0
+    assert bits_equal(a, port.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl))
+    a = qsm.mgpcg_mex(v0, f, m, h, 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl)
+    b = port.mgpcg_mex(v0, f, m, h, 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl)
+    assert bits_equal(a, b), first_diff(a, b)
