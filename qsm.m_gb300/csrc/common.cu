@@ -3,6 +3,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "fp64.cuh"
 
 namespace qsm {
 
@@ -143,6 +144,41 @@ __global__ void cvt_check_k(unsigned long long nfloat, unsigned long long ndoubl
     if (nb) atomicAdd(bad, nb);
 }
 
+// The integer products of fp64.cuh against the hardware multiply: random bit
+// patterns, exponents around one another and around the window's and the range's
+// ends, short significands (ties), zeros.  mw: factors of KMul.
+constexpr int MUL_FACTORS = 12;
+struct MulFactors {
+    KMul<double> k[MUL_FACTORS];
+};
+
+__device__ __forceinline__ bool same_double(double a, double b)
+{
+    return __double_as_longlong(a) == __double_as_longlong(b) || (a != a && b != b);
+}
+
+__global__ void mul_check_k(MulFactors mw, unsigned long long n, unsigned long long *bad)
+{
+    unsigned long long nb = 0;
+    const unsigned long long st = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += st) {
+        uint64_t a = cvt_mix(3 * i), b = cvt_mix(3 * i + 1);
+        const uint64_t m = cvt_mix(3 * i + 2);
+        const uint64_t ends[4] = {540 + (m >> 20) % 8, 1500 + (m >> 20) % 8, 124 + (m >> 20) % 8, 1916 + (m >> 20) % 8};
+        if (m & 1) b = (b & 0x800fffffffffffffull) | ((1023 + ((m >> 1) % 65) - 32) << 52);
+        if ((m & 6) == 2) a = (a & 0x800fffffffffffffull) | (ends[(m >> 8) & 3] << 52);
+        if ((m & 24) == 8) a &= ~0xfffffffull;           // exact products and ties
+        if ((m & 96) == 32) b &= ~0x1fffffffull;
+        if ((m & 896) == 128) a = (a & 0x8000000000000000ull) | ((m >> 30) & 1 ? 0ull : 0x7ff0000000000000ull);
+        const double x = __longlong_as_double((long long)a), y = __longlong_as_double((long long)b);
+        nb += !same_double(xmul(x, y), fp64_mul_hw(x, y));
+        const KMul<double> &k = mw.k[i % MUL_FACTORS];
+        nb += !same_double(k * x, fp64_mul_hw(k.w, x));
+        nb += !same_double(scale2<-3>(x), fp64_mul_hw(0.125, x));
+    }
+    if (nb) atomicAdd(bad, nb);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(RED_BLOCK) lane_dot_kernel(const T *__restrict__ x, const T *__restrict__ y,
                                                              size_t n, T *part, unsigned int *count, double *out)
@@ -158,12 +194,12 @@ __global__ void __launch_bounds__(RED_BLOCK) lane_dot_kernel(const T *__restrict
     for (; i + 3 * RED_LANES < n; i += 4 * RED_LANES) {
         const T x0 = x[i], x1 = x[i + RED_LANES], x2 = x[i + 2 * RED_LANES], x3 = x[i + 3 * RED_LANES];
         const T y0 = y[i], y1 = y[i + RED_LANES], y2 = y[i + 2 * RED_LANES], y3 = y[i + 3 * RED_LANES];
-        acc = acc + x0 * y0;
-        acc = acc + x1 * y1;
-        acc = acc + x2 * y2;
-        acc = acc + x3 * y3;
+        acc = acc + xmul(x0, y0);
+        acc = acc + xmul(x1, y1);
+        acc = acc + xmul(x2, y2);
+        acc = acc + xmul(x3, y3);
     }
-    for (; i < n; i += RED_LANES) acc = acc + x[i] * y[i];
+    for (; i < n; i += RED_LANES) acc = acc + xmul(x[i], y[i]);
     T b = halve_block(sm, tid, acc);
     if (tid == 0) {
         part[blockIdx.x] = b;
@@ -386,6 +422,12 @@ qsm_status qsm_fp_convert_check(qsm_ctx *ctx, unsigned long long *mismatches)
     unsigned long long *bad = (unsigned long long *)ctx->red_out;
     QSM_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), ctx->stream));
     cvt_check_k<<<(unsigned)sms * 8, 256, 0, ctx->stream>>>(1ull << 32, 1ull << 30, bad);
+    QSM_CUDA(cudaGetLastError());
+    const double w[MUL_FACTORS] = {1.0, 0.25, 1.0 / 0.81, 1.0 / 1.44, -6.0, 1.0 / 6.0, 1.9999999999999998, -1.0 / 3.0,
+                                   0.003, 1e-25, 1e60, 0.0};
+    MulFactors mw;
+    for (int i = 0; i < MUL_FACTORS; ++i) mw.k[i] = make_kmul(w[i]);
+    mul_check_k<<<(unsigned)sms * 8, 256, 0, ctx->stream>>>(mw, 1ull << 28, bad);
     QSM_CUDA(cudaGetLastError());
     QSM_CUDA(cudaMemcpyAsync(ctx->host_out, bad, sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
     QSM_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fp64.cuh"
 #include "mg_pack.cuh"
 
 namespace qsm {
@@ -68,6 +69,22 @@ template <typename T> static LapC<T> lap_consts(const double *h)
     c.hz = (T)(1.0 / (h[2] * h[2]));
     c.hh = (T)(-2.0 * (c.hx + c.hy + c.hz));
     return c;
+}
+
+// The same factors where the FP64 pipe bounds the kernel (full SMs): multiplied
+// on the integer pipes (fp64.cuh).
+template <typename T> struct GsK { KMul<T> hx, hy, hz, hh; };
+template <typename T> struct LapK { KMul<T> hx, hy, hz, hh; };
+
+template <typename T> static GsK<T> gs_consts_k(const double *h)
+{
+    const GsC<T> c = gs_consts<T>(h);
+    return GsK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.hh)};
+}
+template <typename T> static LapK<T> lap_consts_k(const double *h)
+{
+    const LapC<T> c = lap_consts<T>(h);
+    return LapK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.hh)};
 }
 
 // ---------------------------------------------------------------------------
@@ -120,7 +137,7 @@ __device__ __forceinline__ void cl_or(uint32_t a, uint32_t v)
 // ---------------------------------------------------------------------------
 
 template <typename T>
-__global__ void gs_color_k(T *v, const T *__restrict__ f, const uint8_t *__restrict__ G, GsC<T> c, Dims d, int par,
+__global__ void gs_color_k(T *v, const T *__restrict__ f, const uint8_t *__restrict__ G, GsK<T> c, Dims d, int par,
                            size_t skip_i)
 {
     const size_t j = 1 + (size_t)blockIdx.y * blockDim.y + threadIdx.y;
@@ -138,7 +155,7 @@ static qsm_status gauss_seidel(qsm_ctx *ctx, T *v, const T *f, const uint8_t *G,
                                int32_t iter, bool rev)
 {
     if (d.nx < 3 || d.ny < 3 || d.nz < 3 || iter <= 0) return QSM_OK;
-    const GsC<T> c = gs_consts<T>(h);
+    const GsK<T> c = gs_consts_k<T>(h);
     const dim3 b(32, 4, 2);
     const dim3 g((unsigned)(((d.nx - 2 + 1) / 2 + 31) / 32), (unsigned)((d.ny - 2 + 3) / 4), (unsigned)((d.nz - 2 + 1) / 2));
     const int par0 = rev ? (int)((d.nx + 1) & 1) : 0;
@@ -164,7 +181,7 @@ static qsm_status gauss_seidel(qsm_ctx *ctx, T *v, const T *f, const uint8_t *G,
 
 template <typename T>
 __global__ void residual_k(T *r, const T *__restrict__ f, const T *__restrict__ x, const uint8_t *__restrict__ G,
-                           LapC<T> c, Dims d)
+                           LapK<T> c, Dims d)
 {
     MG_INTERIOR
     if (!G[l]) return;
@@ -172,7 +189,7 @@ __global__ void residual_k(T *r, const T *__restrict__ f, const T *__restrict__ 
 }
 
 template <typename T>
-__global__ void lapmg_k(T *du, const T *__restrict__ u, const uint8_t *__restrict__ G, LapC<T> c, Dims d)
+__global__ void lapmg_k(T *du, const T *__restrict__ u, const uint8_t *__restrict__ G, LapK<T> c, Dims d)
 {
     MG_INTERIOR
     if (!G[l]) return;
@@ -190,7 +207,7 @@ static qsm_status residual(qsm_ctx *ctx, T *r, const T *f, const T *x, const uin
 {
     const dim3 g = interior_grid3(d);
     if (g.x == 0 || g.y == 0 || g.z == 0) return QSM_OK;
-    residual_k<T><<<g, vox_block(), 0, ctx->stream>>>(r, f, x, G, lap_consts<T>(h), d);
+    residual_k<T><<<g, vox_block(), 0, ctx->stream>>>(r, f, x, G, lap_consts_k<T>(h), d);
     QSM_CUDA(cudaGetLastError());
     return QSM_OK;
 }
@@ -200,7 +217,7 @@ static qsm_status lapmg(qsm_ctx *ctx, T *du, const T *u, const uint8_t *G, const
 {
     const dim3 g = interior_grid3(d);
     if (g.x == 0 || g.y == 0 || g.z == 0) return QSM_OK;
-    lapmg_k<T><<<g, vox_block(), 0, ctx->stream>>>(du, u, G, lap_consts<T>(h), d);
+    lapmg_k<T><<<g, vox_block(), 0, ctx->stream>>>(du, u, G, lap_consts_k<T>(h), d);
     QSM_CUDA(cudaGetLastError());
     return QSM_OK;
 }
@@ -229,7 +246,7 @@ __global__ void restrict_k(T *x2, const T *__restrict__ x, const uint8_t *__rest
                 X(1, 1, 0) + X(0, -1, 1) + X(-1, 0, 1) + X(1, 0, 1) + X(0, 1, 1);
     const T C = X(0, 0, -1) + X(0, -1, 0) + X(-1, 0, 0) + X(1, 0, 0) + X(0, 1, 0) + X(0, 0, 1);
 #undef X
-    x2[l2] = (T)0.015625 * A + (T)0.03125 * B + (T)0.0625 * C + (T)0.125 * x[l];
+    x2[l2] = scale2<-6>(A) + scale2<-5>(B) + scale2<-4>(C) + scale2<-3>(x[l]);
 }
 
 // Fine voxels (i, j, k) in [1, 2(n2-2)]^3: coarse parent i2 = (i+1)/2 and
@@ -258,14 +275,14 @@ __global__ void prolong_k(T *x, const T *__restrict__ x2, const uint8_t *__restr
             const T c0 = x2[l2];
             switch (a + 2 * b + 4 * c) {
             case 0: val = c0; break;
-            case 1: val = (T)0.5 * (c0 + x2[l2 + ox]); break;
-            case 2: val = (T)0.5 * (c0 + x2[l2 + oy]); break;
-            case 4: val = (T)0.5 * (c0 + x2[l2 + oz]); break;
-            case 3: val = (T)0.25 * (c0 + x2[l2 + ox] + x2[l2 + oy] + x2[l2 + ox + oy]); break;
-            case 5: val = (T)0.25 * (c0 + x2[l2 + ox] + x2[l2 + oz] + x2[l2 + ox + oz]); break;
-            case 6: val = (T)0.25 * (c0 + x2[l2 + oy] + x2[l2 + oz] + x2[l2 + oy + oz]); break;
+            case 1: val = scale2<-1>(c0 + x2[l2 + ox]); break;
+            case 2: val = scale2<-1>(c0 + x2[l2 + oy]); break;
+            case 4: val = scale2<-1>(c0 + x2[l2 + oz]); break;
+            case 3: val = scale2<-2>(c0 + x2[l2 + ox] + x2[l2 + oy] + x2[l2 + ox + oy]); break;
+            case 5: val = scale2<-2>(c0 + x2[l2 + ox] + x2[l2 + oz] + x2[l2 + ox + oz]); break;
+            case 6: val = scale2<-2>(c0 + x2[l2 + oy] + x2[l2 + oz] + x2[l2 + oy + oz]); break;
             default:
-                val = (T)0.125 * (c0 + x2[l2 + ox] + x2[l2 + oy] + x2[l2 + oz] + x2[l2 + ox + oy] + x2[l2 + ox + oz] +
+                val = scale2<-3>(c0 + x2[l2 + ox] + x2[l2 + oy] + x2[l2 + oz] + x2[l2 + ox + oy] + x2[l2 + ox + oz] +
                                   x2[l2 + oy + oz] + x2[l2 + ox + oy + oz]);
             }
         }
@@ -494,7 +511,7 @@ __global__ void blist_total_k(const unsigned *__restrict__ segc, const unsigned 
 
 template <typename T>
 __global__ void gs_list_k(T *v, const T *__restrict__ f, const uint32_t *__restrict__ list, unsigned cnt,
-                          uint32_t skip, GsC<T> c, size_t nx, size_t nxny)
+                          uint32_t skip, GsK<T> c, size_t nx, size_t nxny)
 {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= cnt) return;
@@ -511,7 +528,7 @@ __global__ void gs_list_k(T *v, const T *__restrict__ f, const uint32_t *__restr
 constexpr int GS_PER = 4;
 template <typename T>
 __device__ __forceinline__ void gs_list_ilp_body(T *v, const T *__restrict__ f, const uint32_t *__restrict__ list, unsigned cnt,
-                              uint32_t skip, GsC<T> c, size_t nx, size_t nxny, unsigned blk, unsigned nblk)
+                              uint32_t skip, GsK<T> c, size_t nx, size_t nxny, unsigned blk, unsigned nblk)
 {
     const unsigned t0 = blk * blockDim.x + threadIdx.x, st = nblk * blockDim.x;
     size_t l[GS_PER];
@@ -544,7 +561,7 @@ __device__ __forceinline__ void gs_list_ilp_body(T *v, const T *__restrict__ f, 
 
 template <typename T>
 __global__ void gs_list_ilp_k(T *v, const T *__restrict__ f, const uint32_t *__restrict__ list, unsigned cnt,
-                              uint32_t skip, GsC<T> c, size_t nx, size_t nxny)
+                              uint32_t skip, GsK<T> c, size_t nx, size_t nxny)
 {
     gs_list_ilp_body<T>(v, f, list, cnt, skip, c, nx, nxny, blockIdx.x, gridDim.x);
 }
@@ -1711,9 +1728,11 @@ static void plan_coarse_grid(qsm_ctx *ctx, Hier<T> &H)
 
 // The slab solver's kernel for a plan's voxels per thread.
 template <typename T>
-static const void *slab_kernel(int per)
+static const void *slab_kernel(int per, bool soft)
 {
-    return per == 1 ? (const void *)coarse_slab_k<T, 1> : (const void *)coarse_slab_k<T, SL_MAX_PER>;
+    if (sizeof(T) == 8 && soft)
+        return per == 1 ? (const void *)coarse_slab_k<T, 1, GsK<T>> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsK<T>>;
+    return per == 1 ? (const void *)coarse_slab_k<T, 1, GsC<T>> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsC<T>>;
 }
 
 // The slab solver's dynamic shared-memory limit (as cluster_smem_limit).
@@ -1730,9 +1749,9 @@ static size_t slab_smem_limit(qsm_ctx *ctx)
     int maxsm = 0;
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
     size_t l = (size_t)-1;
-    for (int per = 1; per <= SL_MAX_PER; per += SL_MAX_PER - 1) {
+    for (int v = 0; v < 4; ++v) {
         cudaFuncAttributes fa;
-        const void *k = slab_kernel<T>(per);
+        const void *k = slab_kernel<T>(v & 1 ? SL_MAX_PER : 1, v & 2);
         if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || (size_t)maxsm <= fa.sharedSizeBytes ||
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)((size_t)maxsm - fa.sharedSizeBytes)) != cudaSuccess ||
@@ -1800,6 +1819,7 @@ static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, cons
     t.win = ctas > 1 ? (unsigned)((C.d.ny + 1) * ((C.d.nx - 1) / 2) + 2) : 0u;
     t.per = t.cap <= (unsigned)SL_MAX_THREADS ? 1 : SL_MAX_PER;
     t.threads = std::max(64, (int)(((t.cap + t.per - 1) / t.per + 31) / 32 * 32));
+    t.soft = t.cap > SL_SOFT_MIN;
     const SlabLayout lay(t.cap, t.win, ctas, sizeof(T));
     t.smem = lay.bytes;
     if (t.threads > SL_MAX_THREADS || lay.bytes > lim || lay.len > 0xFFFFu) return 0;
@@ -1807,7 +1827,7 @@ static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, cons
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = slab_config<T>(t, at);
     int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, slab_kernel<T>(t.per), &cfg) != cudaSuccess || ncl < 1) {
+    if (cudaOccupancyMaxActiveClusters(&ncl, slab_kernel<T>(t.per, t.soft), &cfg) != cudaSuccess || ncl < 1) {
         cudaGetLastError();
         t.ctas = 0;
         return 0;
@@ -1917,7 +1937,7 @@ template <typename T>
 static qsm_status list_sweeps(qsm_ctx *ctx, T *v, const T *f, uint32_t *const lists[2], const unsigned cnt[2],
                               const double *h, const Dims &d, int32_t iter, bool rev)
 {
-    const GsC<T> c = gs_consts<T>(h);
+    const GsK<T> c = gs_consts_k<T>(h);
     const int par0 = rev ? (int)((d.nx + 1) & 1) : 0;
     const uint32_t skip = rev ? BL_INX2 : BL_I1;
     for (int32_t s = 0; s < iter; ++s)
@@ -1973,7 +1993,7 @@ static qsm_status smooth(qsm_ctx *ctx, const Hier<T> &H, Level<T> &L, int32_t it
 template <typename T>
 __global__ void residual_list_k(T *r, const T *__restrict__ f, const T *__restrict__ x,
                                 const uint32_t *__restrict__ l0, unsigned c0, const uint32_t *__restrict__ l1,
-                                unsigned c1, LapC<T> c, size_t nx, size_t nxny)
+                                unsigned c1, LapK<T> c, size_t nx, size_t nxny)
 {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= c0 + c1) return;
@@ -1986,7 +2006,7 @@ __global__ void residual_list_k(T *r, const T *__restrict__ f, const T *__restri
 template <typename T>
 __device__ __forceinline__ void residual_list_ilp_body(T *r, const T *__restrict__ f, const T *__restrict__ x,
                                     const uint32_t *__restrict__ l0, unsigned c0, const uint32_t *__restrict__ l1,
-                                    unsigned c1, LapC<T> c, size_t nx, size_t nxny, unsigned blk, unsigned nblk)
+                                    unsigned c1, LapK<T> c, size_t nx, size_t nxny, unsigned blk, unsigned nblk)
 {
     const unsigned t0 = blk * blockDim.x + threadIdx.x, st = nblk * blockDim.x;
     size_t l[GS_PER];
@@ -2021,7 +2041,7 @@ __device__ __forceinline__ void residual_list_ilp_body(T *r, const T *__restrict
 template <typename T>
 __global__ void residual_list_ilp_k(T *r, const T *__restrict__ f, const T *__restrict__ x,
                                     const uint32_t *__restrict__ l0, unsigned c0, const uint32_t *__restrict__ l1,
-                                    unsigned c1, LapC<T> c, size_t nx, size_t nxny)
+                                    unsigned c1, LapK<T> c, size_t nx, size_t nxny)
 {
     residual_list_ilp_body<T>(r, f, x, l0, c0, l1, c1, c, nx, nxny, blockIdx.x, gridDim.x);
 }
@@ -2061,14 +2081,14 @@ __device__ __forceinline__ void correct_list_body(T *x, const T *__restrict__ x2
         xv[u] = x[l[u]];
         switch (cs[u]) {
         case 0: val[u] = c0v; break;
-        case 1: val[u] = (T)0.5 * (c0v + x2[q2 + ox]); break;
-        case 2: val[u] = (T)0.5 * (c0v + x2[q2 + oy]); break;
-        case 4: val[u] = (T)0.5 * (c0v + x2[q2 + oz]); break;
-        case 3: val[u] = (T)0.25 * (c0v + x2[q2 + ox] + x2[q2 + oy] + x2[q2 + ox + oy]); break;
-        case 5: val[u] = (T)0.25 * (c0v + x2[q2 + ox] + x2[q2 + oz] + x2[q2 + ox + oz]); break;
-        case 6: val[u] = (T)0.25 * (c0v + x2[q2 + oy] + x2[q2 + oz] + x2[q2 + oy + oz]); break;
+        case 1: val[u] = scale2<-1>(c0v + x2[q2 + ox]); break;
+        case 2: val[u] = scale2<-1>(c0v + x2[q2 + oy]); break;
+        case 4: val[u] = scale2<-1>(c0v + x2[q2 + oz]); break;
+        case 3: val[u] = scale2<-2>(c0v + x2[q2 + ox] + x2[q2 + oy] + x2[q2 + ox + oy]); break;
+        case 5: val[u] = scale2<-2>(c0v + x2[q2 + ox] + x2[q2 + oz] + x2[q2 + ox + oz]); break;
+        case 6: val[u] = scale2<-2>(c0v + x2[q2 + oy] + x2[q2 + oz] + x2[q2 + oy + oz]); break;
         default:
-            val[u] = (T)0.125 * (c0v + x2[q2 + ox] + x2[q2 + oy] + x2[q2 + oz] + x2[q2 + ox + oy] + x2[q2 + ox + oz] +
+            val[u] = scale2<-3>(c0v + x2[q2 + ox] + x2[q2 + oy] + x2[q2 + oz] + x2[q2 + ox + oy] + x2[q2 + ox + oz] +
                                  x2[q2 + oy + oz] + x2[q2 + ox + oy + oz]);
         }
     }
@@ -2104,7 +2124,7 @@ __device__ __forceinline__ void restrict_list_body(T *x2, const T *__restrict__ 
                 X(1, 1, 0) + X(0, -1, 1) + X(-1, 0, 1) + X(1, 0, 1) + X(0, 1, 1);
     const T C = X(0, 0, -1) + X(0, -1, 0) + X(-1, 0, 0) + X(1, 0, 0) + X(0, 1, 0) + X(0, 0, 1);
 #undef X
-    x2[l2] = (T)0.015625 * A + (T)0.03125 * B + (T)0.0625 * C + (T)0.125 * x[l];
+    x2[l2] = scale2<-6>(A) + scale2<-5>(B) + scale2<-4>(C) + scale2<-3>(x[l]);
 }
 
 template <typename T>
@@ -2134,7 +2154,7 @@ static qsm_status level_correct(qsm_ctx *ctx, Level<T> &L, const Level<T> &C, bo
     // from lists where they are long (~36 against ~43 us for a 258^3 level's 5.5M G voxels);
     // the grid kernel stays faster on small levels
     const unsigned n = L.gl[0] ? L.gn[0] + L.gn[1] : 0;
-    if (sizeof(T) != 4 || !clean || n < (1u << 20) || L.n >= ((size_t)1 << 28) || C.d.nx < 3 || C.d.ny < 3 ||
+    if (!clean || n < (1u << 20) || L.n >= ((size_t)1 << 28) || C.d.nx < 3 || C.d.ny < 3 ||
         C.d.nz < 3)
         return prolong<T>(ctx, L.v, C.v, L.G, L.d, C.d, true, clean);
     correct_list_k<T><<<(n + 256 * GS_PER - 1) / (256 * GS_PER), 256, 0, ctx->stream>>>(
@@ -2152,10 +2172,10 @@ static qsm_status level_residual(qsm_ctx *ctx, Level<T> &L)
     if (n == 0 || L.d.nx < 3 || L.d.ny < 3 || L.d.nz < 3) return QSM_OK;
     if (sizeof(T) == 4)
         residual_list_ilp_k<T><<<(n + 256 * GS_PER - 1) / (256 * GS_PER), 256, 0, ctx->stream>>>(
-            L.r, L.f, L.v, L.gl[0], L.gn[0], L.gl[1], L.gn[1], lap_consts<T>(L.h), L.d.nx, L.d.nxny());
+            L.r, L.f, L.v, L.gl[0], L.gn[0], L.gl[1], L.gn[1], lap_consts_k<T>(L.h), L.d.nx, L.d.nxny());
     else
         residual_list_k<T><<<(n + 255) / 256, 256, 0, ctx->stream>>>(L.r, L.f, L.v, L.gl[0], L.gn[0], L.gl[1],
-                                                                     L.gn[1], lap_consts<T>(L.h), L.d.nx, L.d.nxny());
+                                                                     L.gn[1], lap_consts_k<T>(L.h), L.d.nx, L.d.nxny());
     QSM_CUDA(cudaGetLastError());
     return QSM_OK;
 }
@@ -2227,12 +2247,14 @@ static qsm_status coarse_solve(qsm_ctx *ctx, Hier<T> &H, int l, double *scal_dev
         const T *ff = L.f;
         const uint32_t *la = L.gl[0], *lb = L.gl[1];
         Dims dd = L.d;
-        GsC<T> gc = gs_consts<T>(L.h);
+        GsC<T> gh = gs_consts<T>(L.h);
+        GsK<T> gk = gs_consts_k<T>(L.h);
         LapC<T> lc = lap_consts<T>(L.h);
         double tl = tol;
         int *err = H.gb.err, *outer = H.counters;
-        void *args[] = {&vv, &ff, &rr, &la, &lb, &H.sl, &dd, &gc, &lc, &tl, &err, &outer};
-        QSM_CUDA(cudaLaunchKernelExC(&cfg, slab_kernel<T>(H.sl.per), args));
+        void *gc = sizeof(T) == 8 && H.sl.soft ? (void *)&gk : (void *)&gh;
+        void *args[] = {&vv, &ff, &rr, &la, &lb, &H.sl, &dd, gc, &lc, &tl, &err, &outer};
+        QSM_CUDA(cudaLaunchKernelExC(&cfg, slab_kernel<T>(H.sl.per, H.sl.soft), args));
         return QSM_OK;
     }
     if (H.cg_ctas > 0) {
@@ -2414,7 +2436,7 @@ __device__ __forceinline__ T pmad(T x, T y, T z)
     if constexpr (FM)
         return fma(x, y, z);
     else
-        return x * y + z;
+        return xmul(x, y) + z;
 }
 template <typename TP, typename TM>
 __device__ __forceinline__ TP widen(TM v)
@@ -2626,11 +2648,11 @@ __global__ void pcg_p_k(T *__restrict__ p, const T *__restrict__ q, const uint8_
 // q = lapmg(p) on G (interior), then q = -1 * q everywhere; pq = p . q;
 // alpha = rho / pq
 template <typename T, bool FM>
-__device__ __forceinline__ T pcg_lap(const T *__restrict__ p, size_t l, size_t nx, size_t nxny, const LapC<T> &c, T pl)
+__device__ __forceinline__ T pcg_lap(const T *__restrict__ p, size_t l, size_t nx, size_t nxny, const LapK<T> &c, T pl)
 {
     const T sx = p[l - 1] + p[l + 1], sy = p[l - nx] + p[l + nx], sz = p[l - nxny] + p[l + nxny];
     if constexpr (FM)
-        return pmad<true>(c.hz, sz, pmad<true>(c.hy, sy, pmad<true>(c.hx, sx, c.hh * pl)));
+        return pmad<true>(c.hz.w, sz, pmad<true>(c.hy.w, sy, pmad<true>(c.hx.w, sx, c.hh * pl)));
     else
         return c.hh * pl + c.hx * sx + c.hy * sy + c.hz * sz;
 }
@@ -2638,7 +2660,7 @@ __device__ __forceinline__ T pcg_lap(const T *__restrict__ p, size_t l, size_t n
 template <typename T, bool FM>
 __device__ __forceinline__ void pcg_q_body(T *__restrict__ q, const T *__restrict__ p,
                                                      const uint8_t *__restrict__ G, const uint8_t *__restrict__ sk,
-                                                     Segs sg, LapC<T> c, Dims d, T *part, unsigned *count, double *sc, unsigned blk)
+                                                     Segs sg, LapK<T> c, Dims d, T *part, unsigned *count, double *sc, unsigned blk)
 {
     __shared__ T sm[RED_BLOCK];
     const size_t nx = d.nx, ny = d.ny, nxny = d.nxny(), n = d.n();
@@ -2705,7 +2727,7 @@ __device__ __forceinline__ void pcg_q_body(T *__restrict__ q, const T *__restric
 template <typename T, bool FM>
 __global__ void __launch_bounds__(RED_BLOCK) pcg_q_k(T *__restrict__ q, const T *__restrict__ p,
                                                      const uint8_t *__restrict__ G, const uint8_t *__restrict__ sk,
-                                                     Segs sg, LapC<T> c, Dims d, T *part, unsigned *count, double *sc)
+                                                     Segs sg, LapK<T> c, Dims d, T *part, unsigned *count, double *sc)
 {
     pcg_q_body<T, FM>(q, p, G, sk, sg, c, d, part, count, sc, blockIdx.x);
 }
@@ -2842,7 +2864,7 @@ struct PcgState {
     unsigned *count = nullptr;  // their last-block counter
     const uint8_t *sk = nullptr;
     Segs sg{nullptr, nullptr};
-    LapC<TP> lc{};
+    LapK<TP> lc{};
     double res = 0.0, reltol = 0.0;
     int32_t it = 0, maxitcg = 0;
     double tolmg = 0.0;
@@ -2924,7 +2946,7 @@ static qsm_status pcg_setup(qsm_ctx *ctx, PcgState<TP, TM> &S, const Dims &d, co
         QSM_CUDA(cudaGetLastError());
         S.sg = Segs{segk, segcnt};
     }
-    S.lc = lap_consts<TP>(h);
+    S.lc = lap_consts_k<TP>(h);
     // the V-cycle's right-hand side in its own precision; pcg_xr_k refreshes it
     if (!same) cvt_k<TM, TP><<<1216, 256, 0, ctx->stream>>>(H.L[0].f, r, n);
     QSM_CUDA(cudaGetLastError());
@@ -3030,7 +3052,7 @@ struct MvGs {  // one solve's share of a packed colour pass
     const uint32_t *list;
     unsigned cnt, blk0, nblk;
     uint32_t skip;
-    GsC<T> c;
+    GsK<T> c;
     size_t nx, nxny;
 };
 template <typename T>
@@ -3044,7 +3066,7 @@ struct MvLev {  // one solve's level l (residual, restriction onto l + 1, correc
     T *v, *f, *r, *v2, *f2;
     const uint32_t *l0, *l1, *c0l, *c1l;  // level l's and level l+1's G lists
     unsigned n0, n1, m0, m1, blk0, nblk;
-    LapC<T> c;
+    LapK<T> c;
     uint32_t nx, nxny, nx2, nxny2;
     Dims d;
 };
@@ -3080,7 +3102,7 @@ struct MvPcg {  // one solve's PCG vectors and scratch (blocks k RED_NBLK .. (k 
     unsigned *count;
     double *sc;
     size_t n;
-    LapC<TP> lc;
+    LapK<TP> lc;
     Dims dp;
 };
 template <typename TP, typename TM>
@@ -3288,7 +3310,7 @@ static qsm_status pack_sweeps(qsm_ctx *ctx, Hier<T> *const *H, int ns, int l, bo
                 m.list = band ? L.bl[par] : L.gl[par];
                 m.cnt = cnt;
                 m.skip = pass ? (rev ? BL_INX2 : BL_I1) : 0u;
-                m.c = gs_consts<T>(L.h);
+                m.c = gs_consts_k<T>(L.h);
                 m.nx = L.d.nx;
                 m.nxny = L.d.nxny();
                 m.blk0 = blk;
@@ -3333,7 +3355,7 @@ static qsm_status pack_level(qsm_ctx *ctx, Hier<T> *const *H, int ns, int l, int
         m.c1l = C.gl[1];
         m.m0 = C.gn[0];
         m.m1 = C.gn[1];
-        m.c = lap_consts<T>(L.h);
+        m.c = lap_consts_k<T>(L.h);
         m.nx = (uint32_t)L.d.nx;
         m.nxny = (uint32_t)L.d.nxny();
         m.nx2 = (uint32_t)C.d.nx;

@@ -36,6 +36,7 @@
 constexpr int SL_MAX_CTAS = 16;
 constexpr int SL_MAX_THREADS = 1024;
 constexpr int SL_MAX_PER = 2;                     // voxels of each colour per thread
+constexpr unsigned SL_SOFT_MIN = 256;  // FP64 voxels per colour and CTA from which multiplies leave the FP64 pipe
 constexpr unsigned SL_NONE = 0xFFFFFFFFu;         // pos of a voxel no pass updates
 constexpr long long SL_SPIN_LIMIT = 1ll << 20;
 
@@ -50,6 +51,7 @@ struct SlabTab {
     unsigned *pos, *cut;
     int ctas;      // 1, 2, 4, 8 or 16; 0: not used
     int threads, per;
+    bool soft;     // FP64: multiply on the integer pipes
     unsigned cap;  // most voxels of one colour in a chunk
     unsigned win;  // most voxels of one colour within one plane of indices
     size_t smem;
@@ -232,8 +234,8 @@ __device__ __forceinline__ void slab_globals(T (&x)[6], uint32_t g, const T *gv,
 // in FP32 their meta word, SL_ON alone, takes a short way.  FP64 has one way
 // only: a warp with voxels of both kinds would issue the update twice, and an
 // FP64 instruction costs its ~80 cycles whatever lanes it has.
-template <typename T, int PER>
-__device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const SlabCol &C, uint32_t skip, const GsC<T> &c,
+template <typename T, int PER, typename GC>
+__device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const SlabCol &C, uint32_t skip, const GC &c,
                                           const T *gv, int nx, int nxny, uint32_t wait_mb, uint32_t wait_par, bool wait,
                                           int &dead)
 {
@@ -271,11 +273,11 @@ __device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const Slab
     __syncthreads();
 }
 
-template <typename T, int PER>
+template <typename T, int PER, typename GC>
 __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *__restrict__ gf, T *gr,
                                                                 const uint32_t *__restrict__ l0,
                                                                 const uint32_t *__restrict__ l1, SlabTab tab, Dims d,
-                                                                GsC<T> gc, LapC<T> lc, double tol, int *err,
+                                                                GC gc, LapC<T> lc, double tol, int *err,
                                                                 int *outer_out)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -416,7 +418,7 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
 #define SL_PASS(Q, SKIP)                                                                                            \
     do {                                                                                                            \
         if (cn > 1 && tid == 0) sl_arm(mb[Q], bytes[Q]);                                                            \
-        slab_pass<T, PER>(S[Q], col[Q], SKIP, gc, gv, nx, nxny, mb[1 - (Q)], (done[1 - (Q)] - 1) & 1u,              \
+        slab_pass<T, PER, GC>(S[Q], col[Q], SKIP, gc, gv, nx, nxny, mb[1 - (Q)], (done[1 - (Q)] - 1) & 1u,              \
                           done[1 - (Q)] > 0, dead);                                                                 \
         ++done[Q];                                                                                                  \
     } while (0)
