@@ -20,7 +20,7 @@
 //                           forward sweeps + residual + norm) loop in one
 //                           launch: in chunks over a cluster of 1 or 16 CTAs
 //                           (mg_slab.cuh: FP32, and small FP64 grids), over
-//                           every SM with a grid barrier (large FP64 passes),
+//                           every SM (large FP64 passes: mg_flow.cuh),
 //                           in z-slabs or on one CTA (grids without voxel
 //                           lists, packed solves); the norm keeps the lane
 //                           order; no host round trips
@@ -710,15 +710,12 @@ static qsm_status sweeps_cluster(qsm_ctx *ctx, int cn, T *v, const T *f, uint32_
 }
 
 // ---------------------------------------------------------------------------
-// Coarsest level over the whole GPU (mgpcg_mex.c:265-275).  When a colour
-// pass of the coarsest grid is large (a shallow hierarchy, e.g. lbv's on a
-// cropped volume: ~16k FP64 updates per colour), one cluster's 16 SMs are
-// bound by their FP64 pipes (~5 us per pass).  Here one CTA per SM, launched
-// cooperatively so that all are resident, takes every pass over the level's
-// G colour lists and the CTAs meet at a grid barrier between passes.  The
-// residual norm keeps the lane order: CTA b halves the 256-element blocks
-// b, b + grid, ..., CTA 0 halves the 1024 block sums.  Every wait is bounded:
-// a barrier that does not complete within CG_SPIN_LIMIT polls sets the error
+// Coarsest level over the whole GPU (mgpcg_mex.c:265-275) with a grid barrier
+// per colour pass: the form for lists of more voxels than coarse_flow_k's
+// (mg_flow.cuh) CTAs have threads.  One CTA per SM, launched cooperatively so
+// that all are resident, takes every pass over the level's G colour lists and
+// the CTAs meet at a grid barrier between passes.  Every wait is bounded: a
+// barrier that does not complete within CG_SPIN_LIMIT polls sets the error
 // flag, and every CTA leaves at its next barrier.
 // ---------------------------------------------------------------------------
 
@@ -762,32 +759,58 @@ __device__ __forceinline__ bool grid_bar(const GridBar &g, unsigned &k)
     return bad == 0;
 }
 
-// lane-order sum of src[e]^2, e < n (src written before the last barrier);
-// part holds RED_NBLK + 1 values, entries nb .. RED_NBLK - 1 zero
-template <typename T>
-__device__ bool grid_lane_sum(const T *src, unsigned n, T *part, T *red, const GridBar &gb, unsigned &k, T *out)
+// 256-lane blocks that hold elements of an array of n
+__host__ __device__ inline size_t lane_blocks(size_t n)
 {
-    const int tid = threadIdx.x;
-    const unsigned nb = (n + RED_BLOCK - 1) / RED_BLOCK;
-    for (unsigned b = blockIdx.x; b < nb; b += gridDim.x) {
-        const unsigned e = b * RED_BLOCK + tid;
-        const T x = e < n ? __ldcg(src + e) : (T)0;
-        red[tid] = x * x;
-        __syncthreads();
-        for (int st = RED_BLOCK / 2; st > 0; st >>= 1) {
-            if (tid < st) red[tid] = red[tid] + red[tid + st];
-            __syncthreads();
+    return ((n < (size_t)RED_LANES ? n : (size_t)RED_LANES) + RED_BLOCK - 1) / RED_BLOCK;
+}
+
+// sum over N x 32 values in halving order by one warp (value lane + 32 i in x[i]): lane 0 holds it
+template <typename T, int N>
+__device__ __forceinline__ T warp_halve(T (&x)[N])
+{
+#pragma unroll
+    for (int s = N / 2; s > 0; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < s; ++i) x[i] = x[i] + x[i + s];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) x[0] = x[0] + __shfl_down_sync(0xffffffffu, x[0], s);
+    return x[0];
+}
+
+// lane-order sum of src[e]^2, e < n (src written before the last barrier), in
+// every CTA: the 256-lane blocks over the grid's warps, one per turn, then the
+// 1024 block sums by a warp of each CTA; part holds RED_NBLK values, entries
+// lane_blocks(n) .. RED_NBLK - 1 zero
+template <typename T>
+__device__ bool grid_lane_sum(const T *src, size_t n, T *part, T *tot, const GridBar &gb, unsigned &k, T *out)
+{
+    const unsigned nw = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const unsigned nb = (unsigned)lane_blocks(n);
+    for (unsigned b = blockIdx.x * nw + w; b < nb; b += gridDim.x * nw) {
+        T x[RED_BLOCK / 32];
+#pragma unroll
+        for (int i = 0; i < RED_BLOCK / 32; ++i) {
+            T acc = (T)0;
+            for (size_t e = (size_t)b * RED_BLOCK + 32 * i + lane; e < n; e += RED_LANES) {
+                const T y = __ldcg(src + e);
+                acc = acc + y * y;
+            }
+            x[i] = acc;
         }
-        if (tid == 0) part[b] = red[0];
-        __syncthreads();
+        const T s = warp_halve(x);
+        if (lane == 0) part[b] = s;
     }
     if (!grid_bar(gb, k)) return false;
-    if (blockIdx.x == 0) {
-        const T tot = halve_partials(red, tid, part);
-        if (tid == 0) part[RED_NBLK] = tot;
+    if (w == 0) {
+        T x[RED_NBLK / 32];
+#pragma unroll
+        for (int i = 0; i < RED_NBLK / 32; ++i) x[i] = __ldcg(part + 32 * i + lane);
+        const T s = warp_halve(x);
+        if (lane == 0) *tot = s;
     }
-    if (!grid_bar(gb, k)) return false;
-    *out = __ldcg(part + RED_NBLK);
+    __syncthreads();
+    *out = *tot;
     return true;
 }
 
@@ -812,14 +835,14 @@ __global__ void __launch_bounds__(CG_THREADS) coarse_grid_k(T *v, const T *__res
                                                             GsC<T> gc, LapC<T> lc, double tol, GridBar gb, T *part,
                                                             int *outer_out)
 {
-    __shared__ T red[RED_BLOCK];
-    const size_t nx = d.nx, nxny = d.nxny();
-    const unsigned n = (unsigned)d.n(), nb = (n + RED_BLOCK - 1) / RED_BLOCK;
+    __shared__ T tot;
+    const size_t nx = d.nx, nxny = d.nxny(), n = d.n();
+    const unsigned nb = (unsigned)lane_blocks(n);
     if (blockIdx.x == 0)
         for (unsigned b = nb + threadIdx.x; b < RED_NBLK; b += CG_THREADS) part[b] = (T)0;
     unsigned bk = 0;  // barriers passed
     T ff;
-    if (!grid_lane_sum(f, n, part, red, gb, bk, &ff)) return;
+    if (!grid_lane_sum(f, n, part, &tot, gb, bk, &ff)) return;
     const double fn = sizeof(T) == 4 ? (double)sqrtf((float)ff) : sqrt((double)ff);
     const double reltol = tol * fn;
     const int rpar0 = (int)((d.nx + 1) & 1);
@@ -849,7 +872,7 @@ __global__ void __launch_bounds__(CG_THREADS) coarse_grid_k(T *v, const T *__res
         }
         if (!grid_bar(gb, bk)) return;
         T rr;
-        if (!grid_lane_sum(r, n, part, red, gb, bk, &rr)) return;
+        if (!grid_lane_sum(r, n, part, &tot, gb, bk, &rr)) return;
         const double rn = sizeof(T) == 4 ? (double)sqrtf((float)rr) : sqrt((double)rr);
         if (rn < reltol) break;
         if (c0 + c1 == 0) {  // no G voxel: every later outer iteration repeats this one exactly
@@ -1477,6 +1500,7 @@ __global__ void __launch_bounds__(CC_THREADS) coarse_cluster_k(T *gv, const T *_
 }
 
 #include "mg_slab.cuh"
+#include "mg_flow.cuh"
 
 // ---------------------------------------------------------------------------
 // hierarchy and drivers (mgpcg_mex.c:126-332, mg_mex.c:94-207, fmg_mex.c:93-212)
@@ -1517,6 +1541,8 @@ struct Hier {
     bool v0_zero_outside; // level 0's v is +0 outside G whenever a cycle corrects it
     int host_outer;      // outer iterations of the host-driven coarsest solve
     int cg_ctas;         // > 0: the coarsest level runs on this many CTAs, cooperatively (wins over the cluster)
+    int cg_threads;      // > 0: by packets (coarse_flow_k) with that many threads each, else a barrier per pass
+    void *pkt;           // the packets, one per G voxel
     GridBar gb;          // their barrier words (arrival count, error flag)
     void *gpart;         // RED_NBLK + 1 lane-order block sums
     int cc_ctas;         // > 0: the coarsest level runs on a cluster of this many CTAs
@@ -1705,25 +1731,36 @@ static int grid_sweep_ctas(qsm_ctx *ctx)
 }
 
 // The whole-GPU coarsest solver: for large colour passes, or where neither a
-// cluster nor one CTA holds the grid; needs the coarsest level's G lists and
-// cooperative launch.  cg_ctas = one CTA per SM, else 0.
+// cluster nor one CTA holds the grid; needs voxel lists (c0, c1: the coarsest
+// level's) and cooperative launch.  cg_ctas = one CTA per SM, else 0.  Lists of
+// up to FL_THREADS voxels per CTA and colour run by packets (cg_threads),
+// longer ones with a grid barrier per pass.  FP64 solves in ms, packets against
+// barriers (voxels per colour): 38 / 69 (96 x 100 x 40 [7k]), 61 / 113 (190^2 x
+// 110 [11k]), 86 / 156 (224^2 x 128 [16k]), 102 / 188 (120 x 110 x 100 [24k]).
+// Returns the bytes of its tables.
 template <typename T>
-static void plan_coarse_grid(qsm_ctx *ctx, Hier<T> &H)
+static size_t plan_coarse_grid(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1)
 {
     H.cg_ctas = 0;
+    H.cg_threads = 0;
     const Level<T> &C = H.L[H.nl - 1];
-    if (!C.gl[0] || C.d.nx < 3 || C.d.ny < 3 || C.d.nz < 3 || C.n >= (1u << 30)) return;
-    const bool large = C.gn[0] > CG_MIN_PASS || C.gn[1] > CG_MIN_PASS;
-    if (!large && (H.cc_ctas > 0 || H.coarse_in_smem)) return;
-    int coop = 0, sms = 0, per_sm = 0;
+    if (C.d.nx < 3 || C.d.ny < 3 || C.d.nz < 3 || C.n >= (1u << 30)) return 0;
+    const bool large = c0 > CG_MIN_PASS || c1 > CG_MIN_PASS;
+    if (!large && (H.cc_ctas > 0 || H.coarse_in_smem)) return 0;
+    int coop = 0, sms = 0, per_sm = 0, per_sm_flow = 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess || !coop ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, coarse_grid_k<T>, CG_THREADS, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_flow, coarse_flow_k<T>, FL_THREADS, 0) != cudaSuccess ||
         per_sm < 1) {
         cudaGetLastError();
-        return;
+        return 0;
     }
     H.cg_ctas = sms;
+    const unsigned most = (std::max(c0, c1) + (unsigned)sms - 1) / (unsigned)sms;
+    if (per_sm_flow < 1 || most > (unsigned)FL_THREADS) return 0;
+    H.cg_threads = std::max(64, (int)((most + 31) / 32 * 32));
+    return al256(C.n * sizeof(unsigned)) + al256((size_t)(c0 + c1) * sizeof(FlowPkt<T>));
 }
 
 // The slab solver's kernel for a plan's voxels per thread.
@@ -1891,7 +1928,9 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
         for (int p = 0; p < 2; ++p)
             tot += al256((size_t)hc[4 * i + p] * sizeof(uint32_t)) + al256((size_t)hc[4 * i + 2 + p] * sizeof(uint32_t));
     }
-    const size_t sl_bytes = plan_slab<T>(ctx, H, hc[4 * (H.nl - 1) + 2], hc[4 * (H.nl - 1) + 3], hc + 4 * H.nl);
+    const unsigned cc0 = hc[4 * (H.nl - 1) + 2], cc1 = hc[4 * (H.nl - 1) + 3];
+    size_t sl_bytes = plan_slab<T>(ctx, H, cc0, cc1, hc + 4 * H.nl);
+    if (H.sl.ctas == 0) sl_bytes = plan_coarse_grid<T>(ctx, H, cc0, cc1);
     QSM_TRY(dalloc(ctx, &H.lists, tot + 256 + sl_bytes));
     H.sw_ctas = cn;
     char *c = (char *)H.lists;
@@ -1917,17 +1956,16 @@ static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
     }
     QSM_CUDA(cudaGetLastError());
     QSM_TRY(dfree(ctx, segblk));
-    if (H.sl.ctas > 0) {
+    if (H.sl.ctas > 0 || H.cg_threads > 0) {
         const Level<T> &C = H.L[H.nl - 1];
         const unsigned n01 = C.gn[0] + C.gn[1];
         H.sl.pos = (unsigned *)c;
         H.sl.cut = cnt + 4 * H.nl;
+        H.pkt = c + al256(C.n * sizeof(unsigned));
         QSM_CUDA(cudaMemsetAsync(H.sl.pos, 0xFF, C.n * sizeof(unsigned), ctx->stream));
         if (n01) slab_pos_k<<<(n01 + 255) / 256, 256, 0, ctx->stream>>>(H.sl.pos, C.gl[0], C.gn[0], C.gl[1], C.gn[1]);
         QSM_CUDA(cudaGetLastError());
-        return QSM_OK;
     }
-    plan_coarse_grid<T>(ctx, H);
     return QSM_OK;
 }
 
@@ -2268,8 +2306,16 @@ static qsm_status coarse_solve(qsm_ctx *ctx, Hier<T> &H, int l, double *scal_dev
         double tl = tol;
         GridBar gb = H.gb;
         int *outer = H.counters;
-        void *args[] = {&vv, &ff, &rr, &la, &ca, &lb, &cb, &dd, &gc, &lc, &tl, &gb, &part, &outer};
         QSM_CUDA(cudaMemsetAsync(H.gb.count, 0, sizeof(unsigned), ctx->stream));
+        if (H.cg_threads > 0) {
+            const unsigned *pos = H.sl.pos;
+            FlowPkt<T> *pk = (FlowPkt<T> *)H.pkt;
+            void *args[] = {&vv, &ff, &rr, &la, &ca, &lb, &cb, &pos, &pk, &dd, &gc, &lc, &tl, &gb, &part, &outer};
+            QSM_CUDA(cudaLaunchCooperativeKernel((const void *)coarse_flow_k<T>, dim3((unsigned)H.cg_ctas),
+                                                 dim3((unsigned)H.cg_threads), args, 0, ctx->stream));
+            return QSM_OK;
+        }
+        void *args[] = {&vv, &ff, &rr, &la, &ca, &lb, &cb, &dd, &gc, &lc, &tl, &gb, &part, &outer};
         QSM_CUDA(cudaLaunchCooperativeKernel((const void *)coarse_grid_k<T>, dim3((unsigned)H.cg_ctas),
                                              dim3(CG_THREADS), args, 0, ctx->stream));
         return QSM_OK;

@@ -141,20 +141,6 @@ __device__ __forceinline__ bool sl_wait(uint32_t mb, uint32_t parity)
     return false;
 }
 
-// sum over a 256-element block in halving order, one warp, eight elements per
-// lane (element lane + 32 i in x[i]): lane 0 holds it
-template <typename T, int N>
-__device__ __forceinline__ T sl_halve(T (&x)[N])
-{
-#pragma unroll
-    for (int s = N / 2; s > 0; s >>= 1)
-#pragma unroll
-        for (int i = 0; i < s; ++i) x[i] = x[i] + x[i + s];
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) x[0] = x[0] + __shfl_down_sync(0xffffffffu, x[0], s);
-    return x[0];
-}
-
 // lane-order sum of src[e]^2 over e < n <= RED_LANES (src in global memory,
 // written before the last cluster barrier), in every thread of the cluster
 template <typename T>
@@ -171,7 +157,7 @@ __device__ T sl_lane_sum(const T *src, unsigned n, T *blk, T *bc, uint32_t c, ui
         }
 #pragma unroll
         for (int i = 0; i < RED_BLOCK / 32; ++i) x[i] = x[i] * x[i];
-        const T s = sl_halve(x);
+        const T s = warp_halve(x);
         if (lane == 0) cl_st(cl_map(blk, 0) + (uint32_t)(b * sizeof(T)), s);
     }
     cl_sync();
@@ -179,7 +165,7 @@ __device__ T sl_lane_sum(const T *src, unsigned n, T *blk, T *bc, uint32_t c, ui
         T x[RED_NBLK / 32];
 #pragma unroll
         for (int i = 0; i < RED_NBLK / 32; ++i) x[i] = blk[32 * i + lane];  // b >= nb: +0, never written
-        const T s = __shfl_sync(0xffffffffu, sl_halve(x), 0);
+        const T s = __shfl_sync(0xffffffffu, warp_halve(x), 0);
         if (lane < cn) cl_st(cl_map(bc, lane), s);
     }
     cl_sync();

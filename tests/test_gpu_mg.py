@@ -425,3 +425,33 @@ def test_coarse_chunks_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl, kind):
     a = qsm.mgpcg_mex(v0, f, m, h, 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl)
     b = port.mgpcg_mex(v0, f, m, h, 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl)
     assert bits_equal(a, b), first_diff(a, b)
+
+
+@pytest.mark.parametrize("dt", ("float64", "float32"))
+@pytest.mark.parametrize("shape,nl,kind", [((44, 40, 38), 1, "ball"), ((45, 40, 38), 1, "v0"), ((64, 40, 12), 1, "box"),
+                                           ((66, 64, 64), 1, "plates")])
+def test_coarse_packets_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl, kind):
+    """The coarsest solver that passes values between the CTAs of the whole GPU
+    as packets (FP64 passes of more than 6000 voxels; FP32 grids a cluster does
+    not hold): both parities of nx, voxels on the x faces, an initial guess
+    outside the mask, one voxel per CTA up to ~400, and a padded grid of more
+    than 2^18 elements, whose norm sums two elements per lane.  Bit-for-bit
+    against the oracle, whose arithmetic it repeats."""
+    rng = np.random.default_rng(sum(shape))
+    i, j, k = np.ogrid[0:shape[0], 0:shape[1], 0:shape[2]]
+    if kind in ("ball", "v0"):
+        m = sum(((a - (n - 1) / 2) / (0.48 * n)) ** 2 for a, n in zip((i, j, k), shape)) <= 1.0
+    elif kind == "plates":
+        m = (k % 4 == 1) & (i >= 0) & (j > 1)
+    else:
+        m = np.ones(shape, bool)
+    m = np.asfortranarray(np.broadcast_to(m, shape).astype(np.uint8))
+    f = np.asfortranarray((rng.standard_normal(shape) * m).astype(dt))
+    v0 = np.zeros(shape, order="F", dtype=dt)
+    if kind == "v0":
+        v0 = np.asfortranarray((0.1 * rng.standard_normal(shape)).astype(dt))
+    h = [1, 0.9, 1.2]
+    gi = {}
+    a = qsm.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl, info=gi)
+    assert gi["coarse_ctas"] < 0
+    assert bits_equal(a, port.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl))
