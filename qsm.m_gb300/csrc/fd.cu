@@ -5,10 +5,14 @@
 // One thread per voxel.  Every kernel evaluates the per-voxel rule of the
 // reference loop nest it replaces with the same expression and association
 // order; the file is compiled without fused multiply-add, so results are
-// bit-identical to the reference C in FP32 and FP64.  These are single
+// bit-identical to the reference C in FP32 and FP64.  In FP32 these are single
 // sweeps bounded by HBM bandwidth: each reads its inputs once (neighbour
-// re-reads hit L1/L2) and writes each output once.
+// re-reads hit L1/L2) and writes each output once.  In FP64 the FP64 pipe bounds
+// them, so products with 1/h run on the integer pipes (fp64.cuh), a stencil's
+// variants select its operands instead of computing each, and lapw_k forms each
+// difference once.
 #include "common.cuh"
+#include "fp64.cuh"
 
 namespace qsm {
 
@@ -21,7 +25,14 @@ namespace qsm {
     const size_t l = i + nx * j + nxny * k;                                   \
     (void)ny; (void)nz;
 
-template <typename T> struct H3 { T x, y, z; };
+template <typename T> struct H3 { KMul<T> x, y, z; };
+
+// u[l + a] - u[l] (forward), else u[l] - u[l - a]
+template <typename T>
+__device__ __forceinline__ T diff(const T *__restrict__ u, size_t l, size_t a, bool fwd)
+{
+    return u[fwd ? l + a : l] - u[fwd ? l : l - a];
+}
 
 // ---- gradients ----------------------------------------------------------
 
@@ -30,9 +41,9 @@ template <typename T>
 __global__ void gradf_k(T *dx, T *dy, T *dz, const T *__restrict__ u, H3<T> h, Dims d)
 {
     VOXEL_PROLOGUE
-    dx[l] = i + 1 < nx ? h.x * (u[l + 1] - u[l]) : h.x * (u[l] - u[l - 1]);
-    dy[l] = j + 1 < ny ? h.y * (u[l + nx] - u[l]) : h.y * (u[l] - u[l - nx]);
-    dz[l] = k + 1 < nz ? h.z * (u[l + nxny] - u[l]) : h.z * (u[l] - u[l - nxny]);
+    dx[l] = h.x * diff(u, l, 1, i + 1 < nx);
+    dy[l] = h.y * diff(u, l, nx, j + 1 < ny);
+    dz[l] = h.z * diff(u, l, nxny, k + 1 < nz);
 }
 
 // gradb_mex.c:142-229
@@ -40,9 +51,9 @@ template <typename T>
 __global__ void gradb_k(T *dx, T *dy, T *dz, const T *__restrict__ u, H3<T> h, Dims d)
 {
     VOXEL_PROLOGUE
-    dx[l] = i > 0 ? h.x * (u[l] - u[l - 1]) : h.x * (u[l + 1] - u[l]);
-    dy[l] = j > 0 ? h.y * (u[l] - u[l - nx]) : h.y * (u[l + nx] - u[l]);
-    dz[l] = k > 0 ? h.z * (u[l] - u[l - nxny]) : h.z * (u[l + nxny] - u[l]);
+    dx[l] = h.x * diff(u, l, 1, i == 0);
+    dy[l] = h.y * diff(u, l, nx, j == 0);
+    dz[l] = h.z * diff(u, l, nxny, k == 0);
 }
 
 // gradc_mex.c:309-563, including the k = 0 plane overwrite of its
@@ -69,9 +80,10 @@ __global__ void gradfm_k(T *dx, T *dy, T *dz, const T *__restrict__ u, const uin
 {
     VOXEL_PROLOGUE
     if (!G[l]) return;
-    dx[l] = (i + 1 < nx && G[l + 1]) ? h.x * (u[l + 1] - u[l]) : (i > 0 && G[l - 1]) ? h.x * (u[l] - u[l - 1]) : (T)0;
-    dy[l] = (j + 1 < ny && G[l + nx]) ? h.y * (u[l + nx] - u[l]) : (j > 0 && G[l - nx]) ? h.y * (u[l] - u[l - nx]) : (T)0;
-    dz[l] = (k + 1 < nz && G[l + nxny]) ? h.z * (u[l + nxny] - u[l]) : (k > 0 && G[l - nxny]) ? h.z * (u[l] - u[l - nxny]) : (T)0;
+    const bool xf = i + 1 < nx && G[l + 1], yf = j + 1 < ny && G[l + nx], zf = k + 1 < nz && G[l + nxny];
+    dx[l] = xf || (i > 0 && G[l - 1]) ? h.x * diff(u, l, 1, xf) : (T)0;
+    dy[l] = yf || (j > 0 && G[l - nx]) ? h.y * diff(u, l, nx, yf) : (T)0;
+    dz[l] = zf || (k > 0 && G[l - nxny]) ? h.z * diff(u, l, nxny, zf) : (T)0;
 }
 
 // gradbm_mex.c:106-154
@@ -80,9 +92,10 @@ __global__ void gradbm_k(T *dx, T *dy, T *dz, const T *__restrict__ u, const uin
 {
     VOXEL_PROLOGUE
     if (!G[l]) return;
-    dx[l] = (i > 0 && G[l - 1]) ? h.x * (u[l] - u[l - 1]) : (i + 1 < nx && G[l + 1]) ? h.x * (u[l + 1] - u[l]) : (T)0;
-    dy[l] = (j > 0 && G[l - nx]) ? h.y * (u[l] - u[l - nx]) : (j + 1 < ny && G[l + nx]) ? h.y * (u[l + nx] - u[l]) : (T)0;
-    dz[l] = (k > 0 && G[l - nxny]) ? h.z * (u[l] - u[l - nxny]) : (k + 1 < nz && G[l + nxny]) ? h.z * (u[l + nxny] - u[l]) : (T)0;
+    const bool xb = i > 0 && G[l - 1], yb = j > 0 && G[l - nx], zb = k > 0 && G[l - nxny];
+    dx[l] = xb || (i + 1 < nx && G[l + 1]) ? h.x * diff(u, l, 1, !xb) : (T)0;
+    dy[l] = yb || (j + 1 < ny && G[l + nx]) ? h.y * diff(u, l, nx, !yb) : (T)0;
+    dz[l] = zb || (k + 1 < nz && G[l + nxny]) ? h.z * diff(u, l, nxny, !zb) : (T)0;
 }
 
 // gradcm_mex.c:122-186
@@ -117,9 +130,7 @@ template <typename T>
 __global__ void gradf_adj_k(T *du, const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z, H3<T> h, Dims d)
 {
     VOXEL_PROLOGUE
-    const T a = i > 0 ? x[l] - x[l - 1] : x[l + 1] - x[l];
-    const T b = j > 0 ? y[l] - y[l - nx] : y[l + nx] - y[l];
-    const T c = k > 0 ? z[l] - z[l - nxny] : z[l + nxny] - z[l];
+    const T a = diff(x, l, 1, i == 0), b = diff(y, l, nx, j == 0), c = diff(z, l, nxny, k == 0);
     du[l] = h.x * a + h.y * b + h.z * c;
 }
 
@@ -128,9 +139,7 @@ template <typename T>
 __global__ void gradb_adj_k(T *du, const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z, H3<T> h, Dims d)
 {
     VOXEL_PROLOGUE
-    const T a = i + 1 < nx ? x[l + 1] - x[l] : x[l] - x[l - 1];
-    const T b = j + 1 < ny ? y[l + nx] - y[l] : y[l] - y[l - nx];
-    const T c = k + 1 < nz ? z[l + nxny] - z[l] : z[l] - z[l - nxny];
+    const T a = diff(x, l, 1, i + 1 < nx), b = diff(y, l, nx, j + 1 < ny), c = diff(z, l, nxny, k + 1 < nz);
     du[l] = h.x * a + h.y * b + h.z * c;
 }
 
@@ -141,9 +150,10 @@ __global__ void gradfm_adj_k(T *du, const T *__restrict__ x, const T *__restrict
 {
     VOXEL_PROLOGUE
     if (!G[l]) return;
-    const T c = (k > 0 && G[l - nxny]) ? h.z * (z[l] - z[l - nxny]) : (k + 1 < nz && G[l + nxny]) ? h.z * (z[l + nxny] - z[l]) : (T)0;
-    const T b = (j > 0 && G[l - nx]) ? h.y * (y[l] - y[l - nx]) : (j + 1 < ny && G[l + nx]) ? h.y * (y[l + nx] - y[l]) : (T)0;
-    const T a = (i > 0 && G[l - 1]) ? h.x * (x[l] - x[l - 1]) : (i + 1 < nx && G[l + 1]) ? h.x * (x[l + 1] - x[l]) : (T)0;
+    const bool xb = i > 0 && G[l - 1], yb = j > 0 && G[l - nx], zb = k > 0 && G[l - nxny];
+    const T c = zb || (k + 1 < nz && G[l + nxny]) ? h.z * diff(z, l, nxny, !zb) : (T)0;
+    const T b = yb || (j + 1 < ny && G[l + nx]) ? h.y * diff(y, l, nx, !yb) : (T)0;
+    const T a = xb || (i + 1 < nx && G[l + 1]) ? h.x * diff(x, l, 1, !xb) : (T)0;
     du[l] = a + b + c;
 }
 
@@ -154,9 +164,10 @@ __global__ void gradbm_adj_k(T *du, const T *__restrict__ x, const T *__restrict
 {
     VOXEL_PROLOGUE
     if (!G[l]) return;
-    const T a = (i + 1 < nx && G[l + 1]) ? h.x * (x[l + 1] - x[l]) : (i > 0 && G[l - 1]) ? h.x * (x[l] - x[l - 1]) : (T)0;
-    const T b = (j + 1 < ny && G[l + nx]) ? h.y * (y[l + nx] - y[l]) : (j > 0 && G[l - nx]) ? h.y * (y[l] - y[l - nx]) : (T)0;
-    const T c = (k + 1 < nz && G[l + nxny]) ? h.z * (z[l + nxny] - z[l]) : (k > 0 && G[l - nxny]) ? h.z * (z[l] - z[l - nxny]) : (T)0;
+    const bool xf = i + 1 < nx && G[l + 1], yf = j + 1 < ny && G[l + nx], zf = k + 1 < nz && G[l + nxny];
+    const T a = xf || (i > 0 && G[l - 1]) ? h.x * diff(x, l, 1, xf) : (T)0;
+    const T b = yf || (j > 0 && G[l - nx]) ? h.y * diff(y, l, nx, yf) : (T)0;
+    const T c = zf || (k > 0 && G[l - nxny]) ? h.z * diff(z, l, nxny, zf) : (T)0;
     du[l] = a + b + c;
 }
 
@@ -182,16 +193,16 @@ __device__ __forceinline__ T lap_axis(const T *__restrict__ u, const uint8_t *__
                                       size_t n, size_t i, int sel)
 {
     switch (sel) {
-    case 3: return u[l - a] - (T)2 * u[l] + u[l + a];
+    case 3: return u[l - a] - scale2<1>(u[l]) + u[l + a];
     case 2:
         if (i + 3 < n && G[l + 2 * a] && G[l + 3 * a])
-            return (T)2 * u[l] - (T)5 * u[l + a] + (T)4 * u[l + 2 * a] - u[l + 3 * a];
-        if (i + 2 < n && G[l + 2 * a]) return u[l] - (T)2 * u[l + a] + u[l + 2 * a];
+            return scale2<1>(u[l]) - (T)5 * u[l + a] + scale2<2>(u[l + 2 * a]) - u[l + 3 * a];
+        if (i + 2 < n && G[l + 2 * a]) return u[l] - scale2<1>(u[l + a]) + u[l + 2 * a];
         return u[l + a] - u[l];
     case 1:
         if (i >= 3 && G[l - 3 * a] && G[l - 2 * a])
-            return -u[l - 3 * a] + (T)4 * u[l - 2 * a] - (T)5 * u[l - a] + (T)2 * u[l];
-        if (i >= 2 && G[l - 2 * a]) return u[l - 2 * a] - (T)2 * u[l - a] + u[l];
+            return -u[l - 3 * a] + scale2<2>(u[l - 2 * a]) - (T)5 * u[l - a] + scale2<1>(u[l]);
+        if (i >= 2 && G[l - 2 * a]) return u[l - 2 * a] - scale2<1>(u[l - a]) + u[l];
         return u[l - a] - u[l];
     default: return (T)0;
     }
@@ -216,27 +227,80 @@ __global__ void lap1_k(T *du, const T *__restrict__ u, const uint8_t *__restrict
     du[l] = v;
 }
 
-// lapw_mex.c:10-11, :170-187: wrap into [-pi, pi] only when outside.
+// lapw_mex.c:10-11, :170-187: wrap into [-pi, pi] only when outside.  For |x| > 9
+// as the reference has it; up to there fmod(x + pi, 2 pi) is x + pi itself (x <
+// -pi: its magnitude is below 2 pi) or x + pi - 2 pi, exact since x + pi lies in
+// [2 pi, 4 pi): adding pi to the one, subtracting it from the other is one
+// rounding of x + pi + pi or x + pi - 3 pi, the fused multiply-add with 2 pi.
+// FP64 tests run on the encodings, off the FP64 pipe; a NaN is
+// outside no bound.
+__device__ __forceinline__ bool beyond(float x, float b) { return fabsf(x) > b; }
+__device__ __forceinline__ bool beyond(double x, double b)
+{
+    const long long m = __double_as_longlong(x) & 0x7fffffffffffffffll;
+    return m > __double_as_longlong(b) && m <= 0x7ff0000000000000ll;
+}
+
 template <typename T>
 __device__ __forceinline__ T wrap_pi(T x)
 {
     const T pi = (T)3.14159265358979323846;
     const T tau = (T)(2 * 3.14159265358979323846);
-    if (!(x < -pi || x > pi)) return x;
+    if (!beyond(x, pi)) return x;
+    const bool neg = signbit(x), far = beyond(x, (T)9);
     x = x + pi;
-    return x < (T)0 ? fmod(x, tau) + pi : fmod(x, tau) - pi;
+    if (far) return x < (T)0 ? fmod(x, tau) + pi : fmod(x, tau) - pi;
+    return fma(neg ? (T)0.5 : (T)-1.5, tau, x);
 }
 
-// lapw_mex.c:54-167 (interior only)
+// lapw_mex.c:54-167 (interior only).  The six wrapped differences of a voxel are
+// three of its own and three of its lower neighbours': a thread walks up z with
+// LAPW_R rows, so z and most y differences are formed once, and takes the x one
+// of the lane below (lane 0 forms only that: 31 voxels per warp).  FP64: ~8.5
+// FP64 instructions per voxel and 3 per wrapped difference of a warp, against 26
+// and more with six differences per voxel and tests on the FP64 pipe.
+constexpr int LAPW_R = 4, LAPW_TY = 4;
+
 template <typename T>
-__global__ void lapw_k(T *du, const T *__restrict__ u, H3<T> h, Dims d)
+__global__ void __launch_bounds__(32 * LAPW_TY) lapw_k(T *du, const T *__restrict__ u, H3<T> h, Dims d, int kz)
 {
-    VOXEL_PROLOGUE
-    if (i == 0 || j == 0 || k == 0 || i + 1 >= nx || j + 1 >= ny || k + 1 >= nz) return;
-    T v = h.x * (wrap_pi(u[l + 1] - u[l]) - wrap_pi(u[l] - u[l - 1]));
-    v = v + h.y * (wrap_pi(u[l + nx] - u[l]) - wrap_pi(u[l] - u[l - nx]));
-    v = v + h.z * (wrap_pi(u[l + nxny] - u[l]) - wrap_pi(u[l] - u[l - nxny]));
-    du[l] = v;
+    const size_t nx = d.nx, ny = d.ny, nz = d.nz, nxny = nx * ny;
+    const size_t i = (size_t)blockIdx.x * 31 + threadIdx.x;
+    const size_t j0 = 1 + ((size_t)blockIdx.y * LAPW_TY + threadIdx.y) * LAPW_R;
+    const size_t k0 = 1 + (size_t)blockIdx.z * kz, k1 = min(k0 + (size_t)kz, nz - 1);
+    if (j0 + 1 >= ny) return;  // (a whole warp)
+    const bool on = i + 1 < nx, out = on && threadIdx.x > 0;
+    const size_t ic = on ? i : nx - 1;  // lanes past the row read its last voxel
+    const int rows = (int)min((size_t)LAPW_R, ny - 1 - j0);
+    const T *p = u + ic + nx * (j0 - 1) + nxny * k0;
+    T a[LAPW_R + 2], fz[LAPW_R];
+#pragma unroll
+    for (int r = 0; r < LAPW_R + 2; ++r) a[r] = r <= rows + 1 ? p[r * nx] : (T)0;
+#pragma unroll
+    for (int r = 0; r < LAPW_R; ++r) fz[r] = r < rows ? wrap_pi(a[r + 1] - p[(r + 1) * nx - nxny]) : (T)0;
+    for (size_t k = k0; k < k1; ++k, p += nxny) {
+        T n[LAPW_R + 2];
+#pragma unroll
+        for (int r = 0; r < LAPW_R + 2; ++r) n[r] = r <= rows + 1 ? p[r * nx + nxny] : (T)0;
+        T fy = wrap_pi(a[1] - a[0]);
+#pragma unroll
+        for (int r = 0; r < LAPW_R; ++r) {
+            if (r < rows) {  // uniform over the warp
+                const T right = on ? p[(r + 1) * nx + 1] : a[r + 1];
+                const T fx = wrap_pi(right - a[r + 1]);
+                const T bx = __shfl_up_sync(0xffffffffu, fx, 1);
+                const T gy = wrap_pi(a[r + 2] - a[r + 1]), gz = wrap_pi(n[r + 1] - a[r + 1]);
+                T v = h.x * (fx - bx);
+                v = v + h.y * (gy - fy);
+                v = v + h.z * (gz - fz[r]);
+                if (out) du[i + nx * (j0 + r) + nxny * k] = v;
+                fy = gy;
+                fz[r] = gz;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < LAPW_R + 2; ++r) a[r] = n[r];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -245,11 +309,11 @@ __global__ void lapw_k(T *du, const T *__restrict__ u, H3<T> h, Dims d)
 
 template <typename T> static H3<T> inv_h(const double *h, double s)
 {
-    return H3<T>{(T)(s / h[0]), (T)(s / h[1]), (T)(s / h[2])};
+    return H3<T>{make_kmul((T)(s / h[0])), make_kmul((T)(s / h[1])), make_kmul((T)(s / h[2]))};
 }
 template <typename T> static H3<T> inv_h2(const double *h)
 {
-    return H3<T>{(T)(1.0 / (h[0] * h[0])), (T)(1.0 / (h[1] * h[1])), (T)(1.0 / (h[2] * h[2]))};
+    return H3<T>{make_kmul((T)(1.0 / (h[0] * h[0]))), make_kmul((T)(1.0 / (h[1] * h[1]))), make_kmul((T)(1.0 / (h[2] * h[2])))};
 }
 
 enum FdOp {
@@ -281,7 +345,16 @@ static qsm_status launch_fd(qsm_ctx *ctx, FdOp op, const Dims &d, void **a, cons
     case OP_GRADFP_ADJ: gradfp_adj_k<T><<<g, b, 0, s>>>(o0, (const T *)a[1], (const T *)a[2], (const T *)a[3], inv_h<T>(h, -1.0), d); break;
     // Laplacians: a = {d2u, u}
     case OP_LAP1: lap1_k<T><<<g, b, 0, s>>>(o0, (const T *)a[1], G, inv_h2<T>(h), d); break;
-    case OP_LAPW: lapw_k<T><<<g, b, 0, s>>>(o0, (const T *)a[1], inv_h2<T>(h), d); break;
+    case OP_LAPW: {
+        if (d.nx < 3 || d.ny < 3 || d.nz < 3) break;
+        // columns of 16 planes; shorter ones where those would leave SMs without a few blocks each
+        const unsigned gx = (unsigned)((d.nx - 2 + 30) / 31), gy = (unsigned)((d.ny - 2 + LAPW_R * LAPW_TY - 1) / (LAPW_R * LAPW_TY));
+        int kz = 16;
+        while (kz > 2 && (size_t)gx * gy * ((d.nz - 2 + kz - 1) / kz) < 1216) kz /= 2;
+        lapw_k<T><<<dim3(gx, gy, (unsigned)((d.nz - 2 + kz - 1) / kz)), dim3(32, LAPW_TY), 0, s>>>(
+            o0, (const T *)a[1], inv_h2<T>(h), d, kz);
+        break;
+    }
     }
     (void)i1; (void)i2;
     QSM_CUDA(cudaGetLastError());

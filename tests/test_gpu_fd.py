@@ -115,3 +115,31 @@ def test_fd_errors(gpu_ctx, qsm):
     b = np.zeros((4, 4, 4), np.float32, order="F")
     with pytest.raises(TypeError):
         qsm.gradf_mex(b, b.copy(order="F"), b.copy(order="F"), np.zeros((4, 4, 4), order="F"), [1, 1, 1])
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (32, 5, 4), (33, 19, 20), (34, 18, 3), (65, 6, 37), (96, 35, 18)])
+@pytest.mark.parametrize("dt", ("float64", "float32"))
+def test_lapw_tiles_and_wraps_vs_oracle(gpu_ctx, qsm, port, shape, dt):
+    """The wrapped Laplacian's tiles (31 voxels per warp, 4 rows and up to 16
+    planes per thread) at their edges, with phase differences that are exactly
+    pi, one unit beside it, several turns away (the general fmod), and huge.
+    Bit-for-bit against the oracle; infinities and NaNs give NaN where it does."""
+    rng = np.random.default_rng(sum(shape))
+    u = (rng.standard_normal(shape) * 4).astype(dt)
+    pi = np.asarray(np.pi, dtype=dt)
+    pick = rng.integers(0, 12, shape)
+    for q, v in enumerate((0.0, -0.0, pi, -pi, np.nextafter(pi, pi.dtype.type(9)), 3 * pi,
+                           -3 * pi, 50.0, -1e6)):
+        u[pick == q] = v
+    u = np.asfortranarray(u)
+    a, b = np.full(shape, 7.0, dt, order="F"), np.full(shape, 7.0, dt, order="F")
+    qsm.lapw_mex(a, u, [0.7, 1.0, 1.3])
+    port.lapw_mex(b, u, [0.7, 1.0, 1.3])
+    assert bits_equal(a, b), first_diff(a, b)
+    u[1::2, 0::3, 1::2] = np.inf
+    u[0::3, 1::2, 0::2] = np.nan
+    qsm.lapw_mex(a, u, [0.7, 1.0, 1.3])
+    port.lapw_mex(b, u, [0.7, 1.0, 1.3])
+    assert np.array_equal(np.isnan(a), np.isnan(b))
+    ok = ~np.isnan(b)
+    assert bits_equal(np.asfortranarray(np.where(ok, a, 0)), np.asfortranarray(np.where(ok, b, 0)))
