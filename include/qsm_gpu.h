@@ -590,8 +590,8 @@ qsm_status qsm_fp_pipe_rate(qsm_ctx *ctx, qsm_dtype dtype, double *ops_per_s);
  * FP32 <-> FP64 conversions (the mixed-precision PCG's, which keep them off the
  * FP64 pipe) differ from the device's own conversions: all 2^32 floats, and
  * 2^30 doubles, most aimed at rounding ties, subnormal and overflowing float
- * results; and on which its integer-arithmetic FP64 products (fp64.cuh) differ
- * from the device's multiply: 2^28 pairs.  0 on every correct build. */
+ * results; and on which its integer-arithmetic FP64 products and c / sqrt(x)
+ * (fp64.cuh) differ from the device's: 2^28 each.  0 on every correct build. */
 qsm_status qsm_fp_convert_check(qsm_ctx *ctx, unsigned long long *mismatches);
 
 #ifdef __cplusplus

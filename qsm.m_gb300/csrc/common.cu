@@ -144,7 +144,7 @@ __global__ void cvt_check_k(unsigned long long nfloat, unsigned long long ndoubl
     if (nb) atomicAdd(bad, nb);
 }
 
-// The integer products of fp64.cuh against the hardware multiply: random bit
+// The integer products and quotients of fp64.cuh against the hardware: random bit
 // patterns, exponents around one another and around the window's and the range's
 // ends, short significands (ties), zeros.  mw: factors of KMul.
 constexpr int MUL_FACTORS = 12;
@@ -175,6 +175,14 @@ __global__ void mul_check_k(MulFactors mw, unsigned long long n, unsigned long l
         const KMul<double> &k = mw.k[i % MUL_FACTORS];
         nb += !same_double(k * x, fp64_mul_hw(k.w, x));
         nb += !same_double(scale2<-3>(x), fp64_mul_hw(0.125, x));
+        // square roots and quotients: near squares, near powers of four, anything positive
+        uint64_t z = a & 0x7fffffffffffffffull;
+        if (m >> 62) z = (z & 0xfffffffffffffull) | ((1023 - 40 + (m >> 40) % 80) << 52);
+        double v = __longlong_as_double((long long)z);
+        if ((m >> 50) % 3 == 0) v = fp64_mul_hw(v, v);
+        if ((m >> 50) % 7 == 0) v = __longlong_as_double(__double_as_longlong(v) + (long long)((m >> 44) % 3) - 1);
+        nb += !same_double(over_sqrt(k, v), fp64_over_sqrt_hw(k.w, v));
+        nb += above(v, 0.25) != (v > 0.25);
     }
     if (nb) atomicAdd(bad, nb);
 }

@@ -1,4 +1,5 @@
-// FP64 multiplication beside the FP64 pipe.
+// FP64 multiplication, and the quotient of a constant and a square root, beside
+// the FP64 pipe.
 //
 // This GPU has one FP64 unit per SM, which takes ~19 cycles per warp
 // instruction whatever its active lanes (0.50 T operations/s measured, 1/74 of
@@ -141,6 +142,75 @@ __device__ __forceinline__ double scale2(double a)
         return fp64_mul_hw(a, E < 0 ? 1.0 / (double)(1 << (E < 0 ? -E : 0)) : (double)(1 << (E < 0 ? 0 : E)));
     }
     return __hiloint2double((int)(h + ((uint32_t)E << 20)), (int)l);
+}
+
+// x > b for b >= 0 and x not negative (a sum of squares), on the encodings
+__device__ __forceinline__ bool above(float x, float b) { return x > b; }
+__device__ __forceinline__ bool above(double x, double b)
+{
+    const long long m = __double_as_longlong(x);
+    return m > __double_as_longlong(b) && m <= 0x7ff0000000000000ll;  // (no NaN is above)
+}
+
+// c / sqrt(x), each correctly rounded (x > 0): the projections' factor.
+__device__ __forceinline__ float over_sqrt(const KMul<float> &c, float x) { return c.w / sqrtf(x); }
+
+static __device__ __noinline__ double fp64_over_sqrt_hw(double c, double x) { return c / sqrt(x); }
+
+// High 128-bit difference (ah:al) - (bh:bl), arithmetically shifted right by 54.
+__device__ __forceinline__ int64_t sub128_hi(uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl)
+{
+    const uint64_t l = al - bl, h = ah - bh - (al < bl ? 1u : 0u);
+    return (int64_t)((h << 10) | (l >> 54));
+}
+
+// In integers, by Newton's iteration on the residual (Markstein's scheme: an
+// approximation from a short reciprocal, corrected by its exact remainder):
+// r ~ 1/sqrt to 22 bits from rsqrtf; s0 = x r; s1 = s0 + (x - s0^2) r / 2 to ~43
+// bits; s2 = s1 + (x - s1^2) r / 2 to four units in 2^-62, x - s1^2 being exact.
+// A square root is never midway between two doubles, so s2 decides the rounding
+// except within those units of a midpoint m, where m^2 is compared with x
+// exactly.  The quotient c / s follows in the same way from r ~ 1/s.  ~230 cycles
+// per warp and scheduler against ~1200 for the hardware division and square
+// root, which are sequences on the FP64 pipe.
+__device__ __forceinline__ double over_sqrt(const KMul<double> &c, double x)
+{
+    const uint64_t b = (uint64_t)__double_as_longlong(x), ab = (uint64_t)__double_as_longlong(c.w);
+    const uint32_t e = (uint32_t)(b >> 52);
+    if (e - 128u >= 1792u || !c.span || c.s) return fp64_over_sqrt_hw(c.w, x);
+    // x = X 2^-62 4^k, X 2^-62 in [1, 4)
+    const uint32_t odd = (e & 1u) ^ 1u;
+    const uint64_t X = ((b & 0xfffffffffffffull) | (1ull << 52)) << (10 + odd);
+    const float rf = fminf(rsqrtf((float)(uint32_t)(X >> 40) * (1.0f / 4194304.0f)), 1.0f);
+    const uint32_t R = (uint32_t)(rf * 2147483648.0f);  // 2^31 r
+    const uint64_t t0 = ((uint64_t)(uint32_t)(X >> 32) * R) >> 30;
+    const uint32_t S0 = t0 > 0xffffffffull ? 0xffffffffu : (uint32_t)t0;  // 2^31 s0
+    const int64_t D = (int64_t)(X - (uint64_t)S0 * S0);                   // 2^62 (x - s0^2)
+    const uint64_t S1 = ((uint64_t)S0 << 31) + (uint64_t)(((D >> 13) * (int64_t)R) >> 19);  // 2^62 s1
+    const uint64_t S2 = S1 + (uint64_t)((sub128_hi(X >> 2, X << 62, __umul64hi(S1, S1), S1 * S1) * (int64_t)R) >> 40);
+    uint64_t h = S2 >> 10, q = h + (((uint32_t)S2 >> 9) & 1u);
+    if (((uint32_t)S2 & 1023u) - 507u <= 10u) {
+        const uint64_t M = 2 * h + 1, mh = __umul64hi(M, M), ml = M * M, xh = X >> 20, xl = X << 44;
+        q = h + (xh > mh || (xh == mh && xl > ml) ? 1u : 0u);
+    }
+    const uint32_t es = (e + 1023u - odd) >> 1;  // exponent field of s, whose significand is q
+    if (q >> 53) return fp64_over_sqrt_hw(c.w, x);
+    const uint64_t B = q << 11, A = (uint64_t)c.wh << 32 | c.wl;  // significands, 2^63
+    const uint64_t P = (B >> 32) * R + (((uint64_t)(uint32_t)B * R) >> 32);  // 2^62 s r
+    const int64_t E = (int64_t)((1ull << 62) - P);
+    const uint64_t r1 = ((uint64_t)R << 31) + (uint64_t)(((E >> 11) * (int64_t)R) >> 20);  // 2^62 / s to ~42 bits
+    const uint64_t q1 = __umul64hi(A, r1);                                                 // 2^61 c / s
+    const uint64_t q2 = q1 + (uint64_t)((sub128_hi(A >> 3, A << 61, __umul64hi(q1, B), q1 * B) * (int64_t)R) >> 40);
+    const uint32_t ge = (uint32_t)(q2 >> 61), sh = 8 + ge, half = 1u << (sh - 1);
+    h = q2 >> sh;
+    uint64_t m = h + (((uint32_t)q2 >> (sh - 1)) & 1u);
+    if (((uint32_t)q2 & (2 * half - 1)) - (half - 4u) <= 8u) {
+        const uint64_t M = 2 * h + 1, mh = __umul64hi(M, q), ml = M * q, a = A >> 11;
+        const uint64_t xh = a >> (2 + sh), xl = a << (62 - sh);
+        m = h + (xh > mh || (xh == mh && xl > ml) ? 1u : 0u);
+    }
+    const uint64_t er = (ab >> 52) - es + 1022u + ge;
+    return __longlong_as_double((long long)((er << 52) + (m - (1ull << 52))));
 }
 
 #endif  // __CUDACC__

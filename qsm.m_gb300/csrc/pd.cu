@@ -59,6 +59,21 @@ PrimalC<T> make_primal_c(double tau, const double *h)
     return c;
 }
 
+template <typename T>
+static DualK<T> dual_k(const DualC<T> &c)
+{
+    return DualK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.hx2), make_kmul(c.hy2), make_kmul(c.hz2),
+                    make_kmul(c.lhx), make_kmul(c.lhy), make_kmul(c.lhz), make_kmul(c.lhh), make_kmul(c.whx), make_kmul(c.why),
+                    make_kmul(c.whz), make_kmul(c.whh), make_kmul(c.alp0), make_kmul(c.alp1), make_kmul(c.sg), c.alp02, c.alp12};
+}
+template <typename T>
+static PrimalK<T> primal_k(const PrimalC<T> &c)
+{
+    return PrimalK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.lhx), make_kmul(c.lhy), make_kmul(c.lhz),
+                      make_kmul(c.lhh), make_kmul(c.whx), make_kmul(c.why), make_kmul(c.whz), make_kmul(c.whh), make_kmul(c.tt),
+                      make_kmul(c.tau1)};
+}
+
 template DualC<float> make_dual_c<float>(double, const double *, double, double);
 template DualC<double> make_dual_c<double>(double, const double *, double, double);
 template PrimalC<float> make_primal_c<float>(double, const double *);
@@ -153,7 +168,7 @@ static inline dim3 interior_grid(const Dims &d)
 
 // update_dual{d,f} of pd_tgv_mex.c:332-646.
 template <typename T>
-__global__ void tgv_dual_k(PdState<T> s, DualC<T> c, Dims d, const PdCtl *ctl)
+__global__ void tgv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
 {
     if (ctl->done) return;
     INTERIOR_PROLOGUE
@@ -172,10 +187,10 @@ __global__ void tgv_dual_k(PdState<T> s, DualC<T> c, Dims d, const PdCtl *ctl)
     T a1 = p1[l] + c.hx * (chi_[l + 1] - c0) - c.sg * w1[l];
     T a2 = p2[l] + c.hy * (chi_[l + nx] - c0) - c.sg * w2[l];
     T a3 = p3[l] + c.hz * (chi_[l + nxny] - c0) - c.sg * w3[l];
-    T x = a1 * a1 + a2 * a2 + a3 * a3;
-    if (x > c.alp12) {
-        x = c.alp1 / sqrt(x);
-        a1 = a1 * x; a2 = a2 * x; a3 = a3 * x;
+    T x = xmul(a1, a1) + xmul(a2, a2) + xmul(a3, a3);
+    if (above(x, c.alp12)) {
+        x = over_sqrt(c.alp1, x);
+        a1 = xmul(a1, x); a2 = xmul(a2, x); a3 = xmul(a3, x);
     }
     p1[l] = a1; p2[l] = a2; p3[l] = a3;
 
@@ -186,17 +201,17 @@ __global__ void tgv_dual_k(PdState<T> s, DualC<T> c, Dims d, const PdCtl *ctl)
     T b4 = q4[l] + c.hy * (w2[l + nx] - v2);
     T b5 = q5[l] + c.hy2 * (w3[l + nx] - v3) + c.hz2 * (w2[l + nxny] - v2);
     T b6 = q6[l] + c.hz * (w3[l + nxny] - v3);
-    x = b1 * b1 + b4 * b4 + b6 * b6 + (T)2 * (b2 * b2 + b3 * b3 + b5 * b5);
-    if (x > c.alp02) {
-        x = c.alp0 / sqrt(x);
-        b1 = b1 * x; b2 = b2 * x; b3 = b3 * x; b4 = b4 * x; b5 = b5 * x; b6 = b6 * x;
+    x = xmul(b1, b1) + xmul(b4, b4) + xmul(b6, b6) + scale2<1>(xmul(b2, b2) + xmul(b3, b3) + xmul(b5, b5));
+    if (above(x, c.alp02)) {
+        x = over_sqrt(c.alp0, x);
+        b1 = xmul(b1, x); b2 = xmul(b2, x); b3 = xmul(b3, x); b4 = xmul(b4, x); b5 = xmul(b5, x); b6 = xmul(b6, x);
     }
     q1[l] = b1; q2[l] = b2; q3[l] = b3; q4[l] = b4; q5[l] = b5; q6[l] = b6;
 }
 
 // update_primal{d,f} of pd_tgv_mex.c:659-977 (THETA = 1 extragradient).
 template <typename T>
-__global__ void tgv_primal_k(PdState<T> s, PrimalC<T> c, Dims d, const PdCtl *ctl)
+__global__ void tgv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ctl)
 {
     if (ctl->done) return;
     INTERIOR_PROLOGUE
@@ -225,7 +240,7 @@ __global__ void tgv_primal_k(PdState<T> s, PrimalC<T> c, Dims d, const PdCtl *ct
 
 // update_dual{d,f} of pd_tv_mex.c:314-513.
 template <typename T>
-__global__ void tv_dual_k(PdState<T> s, DualC<T> c, Dims d, const PdCtl *ctl)
+__global__ void tv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
 {
     if (ctl->done) return;
     INTERIOR_PROLOGUE
@@ -241,17 +256,17 @@ __global__ void tv_dual_k(PdState<T> s, DualC<T> c, Dims d, const PdCtl *ctl)
     T a1 = p1[l] + c.hx * (chi_[l + 1] - c0);
     T a2 = p2[l] + c.hy * (chi_[l + nx] - c0);
     T a3 = p3[l] + c.hz * (chi_[l + nxny] - c0);
-    T x = a1 * a1 + a2 * a2 + a3 * a3;
-    if (x > c.alp12) {
-        x = c.alp1 / sqrt(x);
-        a1 = a1 * x; a2 = a2 * x; a3 = a3 * x;
+    T x = xmul(a1, a1) + xmul(a2, a2) + xmul(a3, a3);
+    if (above(x, c.alp12)) {
+        x = over_sqrt(c.alp1, x);
+        a1 = xmul(a1, x); a2 = xmul(a2, x); a3 = xmul(a3, x);
     }
     p1[l] = a1; p2[l] = a2; p3[l] = a3;
 }
 
 // update_primal{d,f} of pd_tv_mex.c:524-727.
 template <typename T>
-__global__ void tv_primal_k(PdState<T> s, PrimalC<T> c, Dims d, const PdCtl *ctl)
+__global__ void tv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ctl)
 {
     if (ctl->done) return;
     INTERIOR_PROLOGUE
@@ -379,8 +394,8 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
     const double alpha1 = lam, alpha0 = alpha * lam;
     QSM_TRY(launch_masks(ctx, s.m, s.mi, mask_dev, d));
     QSM_TRY((launch_scale<T, T>(ctx, s.f, (const T *)d2f_dev, sigma, N)));
-    const DualC<T> dc = tgv ? make_dual_c<T>(sigma, h, alpha0, alpha1) : make_dual_c<T>(sigma, h, 0.0, lam);
-    const PrimalC<T> pc = make_primal_c<T>(tau, h);
+    const DualK<T> dc = dual_k(tgv ? make_dual_c<T>(sigma, h, alpha0, alpha1) : make_dual_c<T>(sigma, h, 0.0, lam));
+    const PrimalK<T> pc = primal_k(make_primal_c<T>(tau, h));
     const dim3 g = interior_grid(d), bl = vox_block();
     const bool empty = g.x == 0 || g.y == 0 || g.z == 0;
 
