@@ -178,6 +178,11 @@ __device__ __forceinline__ T halve_partials(T *sm, int tid, const T *part)
     return halve_block(sm, tid, v);
 }
 
+// o[e] = a[0] + ... + a[e - 1] for e < n on the context's stream; tmp holds
+// scan_scratch(n) unsigned (mg.cu)
+size_t scan_scratch(size_t n);
+qsm_status exclusive_scan(qsm_ctx *ctx, const unsigned *a, unsigned *o, size_t n, unsigned *tmp);
+
 // FP32 -> FP64 (exact) and FP64 -> FP32 (round to nearest, ties to even)
 // in integer arithmetic, from the IEEE 754 binary32 / binary64 encodings:
 // the bits of the device's own conversions (a NaN keeps its payload and is

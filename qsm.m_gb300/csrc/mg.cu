@@ -471,8 +471,7 @@ __global__ void scan_add_k(unsigned *o, size_t n, const unsigned *__restrict__ b
     if (e < n) o[e] += bo[e / SCAN_BLK];
 }
 
-// the scratch (unsigned) exclusive_scan needs for n elements
-static size_t scan_scratch(size_t n)
+size_t scan_scratch(size_t n)
 {
     size_t t = 0;
     for (size_t m = n; m > SCAN_BLK;) {
@@ -483,7 +482,7 @@ static size_t scan_scratch(size_t n)
     return t + 16;
 }
 
-static qsm_status exclusive_scan(qsm_ctx *ctx, const unsigned *a, unsigned *o, size_t n, unsigned *tmp)
+qsm_status exclusive_scan(qsm_ctx *ctx, const unsigned *a, unsigned *o, size_t n, unsigned *tmp)
 {
     if (n == 0) return QSM_OK;
     const size_t nb = (n + SCAN_BLK - 1) / SCAN_BLK;

@@ -168,11 +168,8 @@ static inline dim3 interior_grid(const Dims &d)
 
 // update_dual{d,f} of pd_tgv_mex.c:332-646.
 template <typename T>
-__global__ void tgv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
+__device__ __forceinline__ void tgv_dual(const PdState<T> &s, const DualK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
-    if (ctl->done) return;
-    INTERIOR_PROLOGUE
-    if (!s.mi[l]) return;
     const T *chi_ = s.chi_, *eta_ = s.eta_;
     const T *w1 = s.w_, *w2 = s.w_ + N, *w3 = s.w_ + 2 * N;
     T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
@@ -211,11 +208,8 @@ __global__ void tgv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
 
 // update_primal{d,f} of pd_tgv_mex.c:659-977 (THETA = 1 extragradient).
 template <typename T>
-__global__ void tgv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ctl)
+__device__ __forceinline__ void tgv_primal(const PdState<T> &s, const PrimalK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
-    if (ctl->done) return;
-    INTERIOR_PROLOGUE
-    if (!s.m[l]) return;
     const T *nu = s.nu;
     const T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
     const T *q1 = s.q, *q2 = s.q + N, *q3 = s.q + 2 * N, *q4 = s.q + 3 * N, *q5 = s.q + 4 * N, *q6 = s.q + 5 * N;
@@ -240,11 +234,8 @@ __global__ void tgv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ct
 
 // update_dual{d,f} of pd_tv_mex.c:314-513.
 template <typename T>
-__global__ void tv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
+__device__ __forceinline__ void tv_dual(const PdState<T> &s, const DualK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
-    if (ctl->done) return;
-    INTERIOR_PROLOGUE
-    if (!s.mi[l]) return;
     const T *chi_ = s.chi_, *eta_ = s.eta_;
     T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
     const T c0 = chi_[l];
@@ -266,11 +257,8 @@ __global__ void tv_dual_k(PdState<T> s, DualK<T> c, Dims d, const PdCtl *ctl)
 
 // update_primal{d,f} of pd_tv_mex.c:524-727.
 template <typename T>
-__global__ void tv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ctl)
+__device__ __forceinline__ void tv_primal(const PdState<T> &s, const PrimalK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
-    if (ctl->done) return;
-    INTERIOR_PROLOGUE
-    if (!s.m[l]) return;
     const T *nu = s.nu;
     const T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
     const T en = s.eta[l], cn = s.chi[l];
@@ -283,6 +271,120 @@ __global__ void tv_primal_k(PdState<T> s, PrimalK<T> c, Dims d, const PdCtl *ctl
     s.eta[l] = e1; s.chi[l] = c1;
     s.eta_[l] = e1 + (T)1 * (e1 - en);
     s.chi_[l] = c1 + (T)1 * (c1 - cn);
+}
+
+// The two updates of an iteration as kernels: over the interior of the grid, or
+// over the list of its voxels in the mask (FP64: an FP64 instruction takes its
+// slot in the pipe whatever lanes are active, and a row of the grid leaves a
+// third of them off at the mask's edge).
+enum { PD_TGV_DUAL, PD_TGV_PRIMAL, PD_TV_DUAL, PD_TV_PRIMAL };
+template <int STEP, typename T, typename C>
+__device__ __forceinline__ void pd_step(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
+{
+    if constexpr (STEP == PD_TGV_DUAL) tgv_dual<T>(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TGV_PRIMAL) tgv_primal<T>(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TV_DUAL) tv_dual<T>(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TV_PRIMAL) tv_primal<T>(s, c, nx, nxny, N, l);
+}
+
+template <int STEP, typename T, typename C>
+__global__ void pd_grid_k(PdState<T> s, C c, Dims d, const PdCtl *ctl)
+{
+    if (ctl->done) return;
+    INTERIOR_PROLOGUE
+    if (!(STEP == PD_TGV_DUAL || STEP == PD_TV_DUAL ? s.mi[l] : s.m[l])) return;
+    pd_step<STEP>(s, c, nx, nxny, N, l);
+}
+
+template <int STEP, typename T, typename C>
+__global__ void __launch_bounds__(256) pd_list_k(PdState<T> s, C c, Dims d, const uint32_t *__restrict__ list, unsigned cnt,
+                                                 const PdCtl *ctl)
+{
+    if (ctl->done) return;
+    const unsigned t = blockIdx.x * 256 + threadIdx.x;
+    if (t >= cnt) return;
+    pd_step<STEP>(s, c, d.nx, d.nxny(), d.n(), (size_t)list[t]);
+}
+
+// Lists of the interior voxels of mi (q = 0) and m (q = 1) in index order: each
+// row segment of 32 counts its voxels, the counts are scanned, each segment
+// writes its voxels at its offset.
+struct PdLists {
+    uint32_t *l[2];
+    unsigned n[2];
+};
+
+template <bool FILL>
+__global__ void pd_seg_k(PdLists out, unsigned *seg, const uint8_t *__restrict__ mi, const uint8_t *__restrict__ m, Dims d,
+                         size_t nseg)
+{
+    const size_t i = 1 + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t j = 1 + (size_t)blockIdx.y * blockDim.y + threadIdx.y;
+    const size_t k = 1 + (size_t)blockIdx.z * blockDim.z + threadIdx.z;
+    if (j + 1 >= d.ny || k + 1 >= d.nz) return;  // the whole warp (one row)
+    const size_t l = i + d.nx * j + d.nxny() * k;
+    const bool in = i + 1 < d.nx, on[2] = {in && mi[l], in && m[l]};
+    const size_t sg = blockIdx.x + (size_t)gridDim.x * ((j - 1) + (d.ny - 2) * (k - 1));
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const unsigned b = __ballot_sync(0xffffffffu, on[q]);
+        if (!FILL) {
+            if (threadIdx.x == 0) seg[q * nseg + sg] = (unsigned)__popc(b);
+        } else if (on[q]) {
+            out.l[q][seg[q * nseg + sg] - seg[q * nseg] + __popc(b & ((1u << threadIdx.x) - 1u))] = (uint32_t)l;
+        }
+    }
+}
+
+// Builds the lists into *blk (left null where they are not used: FP32, whose
+// kernels HBM bounds, or no memory for them).
+static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t *mi, const uint8_t *m, PdLists *out, void **blk)
+{
+    *blk = nullptr;
+    *out = PdLists{};
+    const dim3 g = interior_grid(d);
+    if (!use || g.x == 0 || g.y == 0 || g.z == 0 || d.n() >= ((size_t)1 << 31)) return QSM_OK;
+    const size_t nseg = (size_t)g.x * (d.ny - 2) * (d.nz - 2);
+    void *seg = nullptr;
+    if (dalloc(ctx, &seg, (4 * nseg + scan_scratch(2 * nseg)) * sizeof(unsigned)) != QSM_OK) {
+        cudaGetLastError();
+        return QSM_OK;
+    }
+    unsigned *segc = (unsigned *)seg, *off = segc + 2 * nseg, *tmp = off + 2 * nseg;
+    pd_seg_k<false><<<g, vox_block(), 0, ctx->stream>>>(PdLists{}, segc, mi, m, d, nseg);
+    QSM_CUDA(cudaGetLastError());
+    QSM_TRY(exclusive_scan(ctx, segc, off, 2 * nseg, tmp));
+    unsigned h[4];  // offsets and counts of the last segment of each list
+    for (int q = 0; q < 2; ++q) {
+        QSM_CUDA(cudaMemcpyAsync(h + q, off + (q + 1) * nseg - 1, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+        QSM_CUDA(cudaMemcpyAsync(h + 2 + q, segc + (q + 1) * nseg - 1, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    QSM_CUDA(cudaStreamSynchronize(ctx->stream));
+    const unsigned n0 = h[0] + h[2], n1 = h[1] + h[3] - n0;
+    if (dalloc(ctx, blk, ((size_t)n0 + n1 + 2) * sizeof(uint32_t)) != QSM_OK) {
+        cudaGetLastError();
+        *blk = nullptr;
+        return dfree(ctx, seg);
+    }
+    uint32_t *l = (uint32_t *)*blk;
+    *out = PdLists{{l, l + n0}, {n0, n1}};
+    pd_seg_k<true><<<g, vox_block(), 0, ctx->stream>>>(*out, off, mi, m, d, nseg);
+    QSM_CUDA(cudaGetLastError());
+    return dfree(ctx, seg);
+}
+
+template <int STEP, typename T, typename C>
+static void launch_step(qsm_ctx *ctx, const PdState<T> &s, const C &c, const Dims &d, const PdLists &ls, bool lists,
+                        const PdCtl *ctl)
+{
+    const int q = STEP == PD_TGV_DUAL || STEP == PD_TV_DUAL ? 0 : 1;
+    if constexpr (sizeof(T) == 8) {
+        if (lists) {
+            if (ls.n[q]) pd_list_k<STEP, T, C><<<(ls.n[q] + 255) / 256, 256, 0, ctx->stream>>>(s, c, d, ls.l[q], ls.n[q], ctl);
+            return;
+        }
+    }
+    pd_grid_k<STEP, T, C><<<interior_grid(d), vox_block(), 0, ctx->stream>>>(s, c, d, ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -396,8 +498,11 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
     QSM_TRY((launch_scale<T, T>(ctx, s.f, (const T *)d2f_dev, sigma, N)));
     const DualK<T> dc = dual_k(tgv ? make_dual_c<T>(sigma, h, alpha0, alpha1) : make_dual_c<T>(sigma, h, 0.0, lam));
     const PrimalK<T> pc = primal_k(make_primal_c<T>(tau, h));
-    const dim3 g = interior_grid(d), bl = vox_block();
+    const dim3 g = interior_grid(d);
     const bool empty = g.x == 0 || g.y == 0 || g.z == 0;
+    PdLists ls;
+    void *lblk = nullptr;
+    QSM_TRY(pd_lists(ctx, sizeof(T) == 8, d, s.mi, s.m, &ls, &lblk));
 
     cudaEvent_t e0, e1;
     QSM_CUDA(cudaEventCreate(&e0));
@@ -416,11 +521,11 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
         }
         if (!empty) {
             if (tgv) {
-                tgv_dual_k<T><<<g, bl, 0, ctx->stream>>>(s, dc, d, ctl);
-                tgv_primal_k<T><<<g, bl, 0, ctx->stream>>>(s, pc, d, ctl);
+                launch_step<PD_TGV_DUAL>(ctx, s, dc, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TGV_PRIMAL>(ctx, s, pc, d, ls, lblk != nullptr, ctl);
             } else {
-                tv_dual_k<T><<<g, bl, 0, ctx->stream>>>(s, dc, d, ctl);
-                tv_primal_k<T><<<g, bl, 0, ctx->stream>>>(s, pc, d, ctl);
+                launch_step<PD_TV_DUAL>(ctx, s, dc, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TV_PRIMAL>(ctx, s, pc, d, ls, lblk != nullptr, ctl);
             }
             QSM_CUDA(cudaGetLastError());
         }
@@ -452,6 +557,7 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
         info->active_voxels = (uint64_t)(d.nx > 2 ? d.nx - 2 : 0) * (d.ny > 2 ? d.ny - 2 : 0) * (d.nz > 2 ? d.nz - 2 : 0);
         info->tile[0] = info->tile[1] = info->tile[2] = 0;
     }
+    if (lblk) QSM_TRY(dfree(ctx, lblk));
     QSM_TRY(dfree(ctx, blk));
     return QSM_OK;
 }

@@ -82,7 +82,8 @@ __device__ __forceinline__ void pd_finish(PdCtl *ctl, const double *s, double to
 __device__ __forceinline__ void mon_terms(double x, double x0, double e, double e0, double &a, double &b,
                                           double &c, double &dd)
 {
-    a = x * x; b = e * e; c = (x - x0) * (x - x0); dd = (e - e0) * (e - e0);
+    const double dx = x - x0, de = e - e0;
+    a = xmul(x, x); b = xmul(e, e); c = xmul(dx, dx); dd = xmul(de, de);
 }
 __device__ __forceinline__ void mon_terms(float x, float x0, float e, float e0, double &a, double &b,
                                           double &c, double &dd)

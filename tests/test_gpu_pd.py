@@ -269,3 +269,26 @@ def test_fused_large_volume_matches_plain(gpu_ctx, qsm):
     a = qsm.pd_tv_mex(d2f, mask, [1, 1, 1], 0.003, 0.0, 12, fused=True)
     b = qsm.pd_tv_mex(d2f, mask, [1, 1, 1], 0.003, 0.0, 12)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape,kind", [((3, 3, 3), "full"), ((35, 5, 4), "full"), ((33, 34, 9), "dots"), ((66, 7, 12), "faces"),
+                                        ((20, 20, 20), "none"), ((40, 36, 30), "ball")])
+def test_pd_plain_voxel_lists(gpu_ctx, qsm, port, shape, kind):
+    """The plain FP64 path runs from lists of the mask's interior voxels: masks
+    that fill the grid, hold single voxels (whose neighbours' interior mask is set
+    where they are not), touch only its faces, or nothing.  Bit-for-bit against
+    the oracle, TGV and TV."""
+    rng = np.random.default_rng(sum(shape))
+    i, j, k = np.ogrid[0:shape[0], 0:shape[1], 0:shape[2]]
+    m = {"full": np.ones(shape, bool), "dots": rng.random(shape) < 0.6, "none": np.zeros(shape, bool),
+         "faces": (i < 2) | (j == shape[1] - 1) | (k < 3) | (i > shape[0] - 3),
+         "ball": sum(((a - (n - 1) / 2) / (0.45 * n)) ** 2 for a, n in zip((i, j, k), shape)) <= 1}[kind]
+    m = np.asfortranarray(np.broadcast_to(m, shape).astype(np.uint8))
+    f = np.asfortranarray(rng.standard_normal(shape) * 0.05)
+    h = [1.0, 0.9, 1.4]
+    a = qsm.pd_tgv_mex(f, m, h, 0.003, 2.0, 0.0, 23)
+    b = port.pd_tgv_mex(f, m, h, 0.003, 2.0, 0.0, 23)
+    assert bits_equal(a, b), first_diff(a, b)
+    a = qsm.pd_tv_mex(f, m, h, 0.003, 0.0, 23)
+    b = port.pd_tv_mex(f, m, h, 0.003, 0.0, 23)
+    assert bits_equal(a, b), first_diff(a, b)
