@@ -512,7 +512,7 @@ qsm_status rebuild(qsm_session *s)
             a.gbase = s->d_gbase;
             a.start = j->start;
             a.maxiter = j->maxiter;
-            if (pd_volume_launch(ctx, st, j->v, ((i + 1) % 10) == 0, a, j->tol, i, i % kPhases) != QSM_OK)
+            if (pd_volume_launch(ctx, st, j->v, ((i + 1) % 10) == 0, a, j->tol, i, i % kPhases, i > 0) != QSM_OK)
                 ce = cudaErrorLaunchFailure;
         }
     }
@@ -701,7 +701,10 @@ qsm_status qsm_session_submit_pd(qsm_session *s, int32_t tgv, qsm_dtype dt, cons
     qsm_status st = pd_volume_init(ctx, &j->v, tgv != 0, d, dt, sf.dev, (const uint8_t *)sm.dev, vsz, lam, alpha);
     if (st == QSM_OK) st = pd_volume_tune(ctx, &j->v, maxiter);
     // a volume small enough to be packed runs the packed kernels, which have no TMA form
-    if (st == QSM_OK && variant(j->v.var).tma && j->v.tl[j->v.var].nact < s->solo_tiles) j->v.var = kTmaFallback;
+    if (st == QSM_OK && variant(j->v.var).tma && j->v.tl[j->v.var].nact < s->solo_tiles) {
+        j->v.var = kTmaFallback;
+        st = pd_volume_tiles(ctx, &j->v, j->v.var);
+    }
     stage_out(ctx, sf, false);
     stage_out(ctx, sm, false);
     if (st != QSM_OK) {

@@ -87,11 +87,13 @@ __global__ void __launch_bounds__(TX * TY, MINB)
 tgv_fused_k(FusedArgs s, DualC<float> dc, PrimalC<float> pc, Dims d, double tol, uint32_t it)
 {
     extern __shared__ double shd_raw[];  // the dual (reused for the monitor reduction)
+    const unsigned tile = __ldg(s.tiles + blockIdx.x);
+    pdl_begin();
     if (s.ctl->done) return;
     const uint32_t itn = launch_iter(s, it);
     if (!itn) return;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    tile_tgv<TX, TY, TZ>(s, dc, pc, d, s.tiles[blockIdx.x], CHECK, (float *)shd_raw, acc);
+    tile_tgv<TX, TY, TZ>(s, dc, pc, d, tile, CHECK, (float *)shd_raw, acc);
     if (CHECK) monitor_reduce<TX * TY>(s, shd_raw, acc, tol, itn);
 }
 
@@ -104,11 +106,13 @@ __global__ void __launch_bounds__(TX * TY, MINB)
 tv_fused_k(FusedArgs s, DualC<float> dc, PrimalC<float> pc, Dims d, double tol, uint32_t it)
 {
     extern __shared__ double shd_raw[];  // the dual (reused for the monitor reduction)
+    const unsigned tile = __ldg(s.tiles + blockIdx.x);
+    pdl_begin();
     if (s.ctl->done) return;
     const uint32_t itn = launch_iter(s, it);
     if (!itn) return;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    tile_tv<TX, TY, TZ>(s, dc, pc, d, s.tiles[blockIdx.x], CHECK, (float *)shd_raw, acc);
+    tile_tv<TX, TY, TZ>(s, dc, pc, d, tile, CHECK, (float *)shd_raw, acc);
     if (CHECK) monitor_reduce<TX * TY>(s, shd_raw, acc, tol, itn);
 }
 
@@ -144,15 +148,15 @@ size_t variant_smem(int v, bool tgv)
 }
 
 template <int TX, int TY, int TZ, int MINB>
-static void launch_t(cudaStream_t st, bool tgv, bool chk, unsigned nact, const FusedArgs &s, const DualC<float> &dc,
+static void launch_t(cudaStream_t st, bool chain, bool tgv, bool chk, unsigned nact, const FusedArgs &s, const DualC<float> &dc,
                      const PrimalC<float> &pc, const Dims &d, double tol, uint32_t it, size_t smem)
 {
     if (tgv) {
-        if (chk) tgv_fused_k<TX, TY, TZ, MINB, true><<<nact, TX * TY, smem, st>>>(s, dc, pc, d, tol, it);
-        else tgv_fused_k<TX, TY, TZ, MINB, false><<<nact, TX * TY, smem, st>>>(s, dc, pc, d, tol, it);
+        launch_iteration(chk ? tgv_fused_k<TX, TY, TZ, MINB, true> : tgv_fused_k<TX, TY, TZ, MINB, false>, chain, nact, TX * TY,
+                         smem, st, s, dc, pc, d, tol, it);
     } else {
-        if (chk) tv_fused_k<TX, TY, TZ, MINB, true><<<nact, TX * TY, smem, st>>>(s, dc, pc, d, tol, it);
-        else tv_fused_k<TX, TY, TZ, MINB, false><<<nact, TX * TY, smem, st>>>(s, dc, pc, d, tol, it);
+        launch_iteration(chk ? tv_fused_k<TX, TY, TZ, MINB, true> : tv_fused_k<TX, TY, TZ, MINB, false>, chain, nact, TX * TY,
+                         smem, st, s, dc, pc, d, tol, it);
     }
 }
 
@@ -174,18 +178,18 @@ bool variant_ok(const PdVolume &v, int var)
 // tm: the volume's TMA maps of this iteration (TMA variants)
 static qsm_status launch_variant(qsm_ctx *ctx, cudaStream_t st, int v, bool tgv, bool chk, unsigned nact,
                                  const FusedArgs &s, const DualC<float> &dc, const PrimalC<float> &pc, const Dims &d,
-                                 double tol, uint32_t it, const TmaMaps *tm)
+                                 double tol, uint32_t it, const TmaMaps *tm, bool chain)
 {
     const size_t sm = variant_smem(v, tgv);
     if (kVariants[v].tma && !tm) return QSM_ERR_ARG;
     if (kVariants[v].stream)
         return stream_launch(ctx, st, kVariants[v].tx, kVariants[v].ty, kVariants[v].tz, tgv, chk, nact, s, dc, pc, d,
-                             tol, it, kVariants[v].tma ? tm : nullptr);
+                             tol, it, kVariants[v].tma ? tm : nullptr, chain);
     switch (v) {
-    case 0: launch_t<32, 8, 4, 4>(st, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
-    case 1: launch_t<32, 8, 2, 4>(st, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
-    case 2: launch_t<32, 4, 4, 8>(st, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
-    case 3: launch_t<32, 16, 2, 2>(st, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
+    case 0: launch_t<32, 8, 4, 4>(st, chain, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
+    case 1: launch_t<32, 8, 2, 4>(st, chain, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
+    case 2: launch_t<32, 4, 4, 8>(st, chain, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
+    case 3: launch_t<32, 16, 2, 2>(st, chain, tgv, chk, nact, s, dc, pc, d, tol, it, sm); break;
     default: return QSM_ERR_ARG;
     }
     QSM_CUDA(cudaGetLastError());
@@ -200,10 +204,10 @@ static const TmaMaps *volume_maps(const PdVolume &v, int var, uint32_t rot)
 }
 
 qsm_status pd_volume_launch(qsm_ctx *ctx, cudaStream_t st, const PdVolume &v, bool chk, const FusedArgs &s,
-                            double tol, uint32_t it, uint32_t rot)
+                            double tol, uint32_t it, uint32_t rot, bool chain)
 {
     return launch_variant(ctx, st, v.var, v.tgv, chk, v.tl[v.var].nact, s, v.dc, v.pc, v.d, tol, it,
-                          volume_maps(v, v.var, rot));
+                          volume_maps(v, v.var, rot), chain);
 }
 
 static qsm_status set_all_smem(qsm_ctx *ctx)
@@ -281,11 +285,11 @@ Layout layout(bool tgv, const Dims &d)
         L.ntiles_total += nb;
         L.nblk_max = std::max(L.nblk_max, nb);
     }
-    // 3 primal buffers + 2 dual buffers + f, 3 mask arrays, tile lists, tile flags,
+    // 3 primal buffers + 2 dual buffers + f, 3 mask arrays, tile lists,
     // monitor partials, counter + control block
     L.bytes = 3 * (L.pa + L.pb) + 2 * (L.da + L.db + L.dc) + L.stride + 3 * L.mstride +
               (L.ntiles_total + 64) * sizeof(unsigned) +
-              (L.nblk_max + 64) + 256 + 4 * (L.nblk_max + 1) * sizeof(double) + 1024;
+              256 + 4 * (L.nblk_max + 1) * sizeof(double) + 1024;
     return L;
 }
 }  // namespace
@@ -316,8 +320,6 @@ qsm_status pd_volume_init(qsm_ctx *ctx, PdVolume *v, bool tgv, const Dims &d, qs
     c += 3 * L.mstride;
     unsigned *tiles_base = (unsigned *)c;
     c += (L.ntiles_total + 64) * sizeof(unsigned);
-    uint8_t *tflag = (uint8_t *)c;
-    c += L.nblk_max + 64;
     c = (char *)(((uintptr_t)c + 255) & ~(uintptr_t)255);
     v->part = (double *)c;
     c += 4 * (L.nblk_max + 1) * sizeof(double);
@@ -337,8 +339,6 @@ qsm_status pd_volume_init(qsm_ctx *ctx, PdVolume *v, bool tgv, const Dims &d, qs
     else
         QSM_TRY((launch_scale<float, double>(ctx, v->f, (const double *)d2f, sigma, N)));
 
-    // active tiles of every variant, ascending (fixed order of the monitor partials)
-    const size_t ix = d.nx > 2 ? d.nx - 2 : 0, iy = d.ny > 2 ? d.ny - 2 : 0, iz = d.nz > 2 ? d.nz - 2 : 0;
     unsigned *tp = tiles_base;
     for (int k = 0; k < kNumVariants; ++k) {
         TileList &tl = v->tl[k];
@@ -346,30 +346,8 @@ qsm_status pd_volume_init(qsm_ctx *ctx, PdVolume *v, bool tgv, const Dims &d, qs
         tl.gx = L.gx[k];
         tl.gy = L.gy[k];
         tl.gz = L.gz[k];
-        const size_t nb = (size_t)tl.gx * tl.gy * tl.gz;
         tl.dev = tp;
-        tp += nb;
-        if (!nb) continue;
-        tile_flags_k<<<(unsigned)nb, 256, 0, ctx->stream>>>(tflag, v->mm, d, tl.gx, tl.gy, kVariants[k].tx,
-                                                            kVariants[k].ty, kVariants[k].tz);
-        QSM_CUDA(cudaGetLastError());
-        std::vector<uint8_t> hf(nb);
-        QSM_CUDA(cudaMemcpyAsync(hf.data(), tflag, nb, cudaMemcpyDeviceToHost, ctx->stream));
-        QSM_CUDA(cudaStreamSynchronize(ctx->stream));
-        std::vector<unsigned> ht;
-        ht.reserve(nb);
-        for (size_t t = 0; t < nb; ++t) {
-            if (!hf[t]) continue;
-            ht.push_back((unsigned)t);
-            const size_t ttx = t % tl.gx, tty = (t / tl.gx) % tl.gy, ttz = t / ((size_t)tl.gx * tl.gy);
-            tl.active_vox += std::min((size_t)kVariants[k].tx, ix - ttx * kVariants[k].tx) *
-                             std::min((size_t)kVariants[k].ty, iy - tty * kVariants[k].ty) *
-                             std::min((size_t)kVariants[k].tz, iz - ttz * kVariants[k].tz);
-        }
-        tl.nact = (unsigned)ht.size();
-        if (!ht.empty())
-            QSM_CUDA(cudaMemcpyAsync(tl.dev, ht.data(), ht.size() * sizeof(unsigned), cudaMemcpyHostToDevice, ctx->stream));
-        QSM_CUDA(cudaStreamSynchronize(ctx->stream));
+        tp += (size_t)tl.gx * tl.gy * tl.gz;
     }
     v->dc = tgv ? make_dual_c<float>(sigma, h, alpha * lam, lam) : make_dual_c<float>(sigma, h, 0.0, lam);
     v->pc = make_primal_c<float>(tau, h);
@@ -400,6 +378,40 @@ qsm_status pd_volume_init(qsm_ctx *ctx, PdVolume *v, bool tgv, const Dims &d, qs
         }
         v->maps.swap(maps);
     }
+    return QSM_OK;
+}
+
+// Active tiles in ascending order: neighbouring tiles run at about the same time
+// and share their halos in L2 (sorted by work, so that the last CTAs of a launch are
+// light ones, an iteration takes 101.6 instead of 97.3 us at 224x224x128).
+qsm_status pd_volume_tiles(qsm_ctx *ctx, PdVolume *v, int var)
+{
+    TileList &tl = v->tl[var];
+    const size_t nb = (size_t)tl.gx * tl.gy * tl.gz;
+    if (tl.built || !nb) return QSM_OK;
+    const Variant &x = kVariants[var];
+    const Dims &d = v->d;
+    uint8_t *flag = (uint8_t *)v->part;  // scratch: the monitors' partials, written before they are read
+    tile_flags_k<<<(unsigned)nb, 256, 0, ctx->stream>>>(flag, v->mm, d, tl.gx, tl.gy, x.tx, x.ty, x.tz);
+    QSM_CUDA(cudaGetLastError());
+    std::vector<uint8_t> hf(nb);
+    std::vector<unsigned> ht;
+    QSM_CUDA(cudaMemcpyAsync(hf.data(), flag, nb, cudaMemcpyDeviceToHost, ctx->stream));
+    QSM_CUDA(cudaStreamSynchronize(ctx->stream));
+    ht.reserve(nb);
+    const size_t ix = d.nx - 2, iy = d.ny - 2, iz = d.nz - 2;
+    for (size_t t = 0; t < nb; ++t) {
+        if (!hf[t]) continue;
+        ht.push_back((unsigned)t);
+        const size_t ttx = t % tl.gx, tty = (t / tl.gx) % tl.gy, ttz = t / ((size_t)tl.gx * tl.gy);
+        tl.active_vox += std::min((size_t)x.tx, ix - ttx * x.tx) * std::min((size_t)x.ty, iy - tty * x.ty) *
+                         std::min((size_t)x.tz, iz - ttz * x.tz);
+    }
+    tl.nact = (unsigned)ht.size();
+    tl.built = true;
+    if (!ht.empty())
+        QSM_CUDA(cudaMemcpyAsync(tl.dev, ht.data(), ht.size() * sizeof(unsigned), cudaMemcpyHostToDevice, ctx->stream));
+    QSM_CUDA(cudaStreamSynchronize(ctx->stream));
     return QSM_OK;
 }
 
@@ -438,7 +450,7 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
     if (force && *force) {
         v->var = std::min(std::max(atoi(force), 0), kNumVariants - 1);
         if (!variant_ok(*v, v->var)) v->var = kTmaFallback;
-        return QSM_OK;
+        return pd_volume_tiles(ctx, v, v->var);
     }
     const TuneKey key((int)v->tgv, v->d.nx, v->d.ny, v->d.nz);
     {
@@ -447,10 +459,11 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
         auto itk = g_tuned.find(key);
         if (itk != g_tuned.end() && variant_ok(*v, itk->second)) {
             v->var = itk->second;
-            return QSM_OK;
+            return pd_volume_tiles(ctx, v, v->var);
         }
     }
     v->var = 0;
+    QSM_TRY(pd_volume_tiles(ctx, v, 0));
     if (v->tl[0].nact == 0 || maxiter < 20) return QSM_OK;
     // time each variant over a few iterations on this problem, then reset the state
     cudaEvent_t t0, t1;
@@ -459,17 +472,24 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
     float best = 1e30f;
     for (int k = 0; k < kNumVariants; ++k) {
         if (!variant_ok(*v, k)) continue;
+        QSM_TRY(pd_volume_tiles(ctx, v, k));
         for (uint32_t it = 0; it < 2; ++it)
             QSM_TRY(launch_variant(ctx, ctx->stream, k, v->tgv, false, v->tl[k].nact, pd_volume_args(*v, k, it),
-                                   v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it)));
-        QSM_CUDA(cudaEventRecord(t0, ctx->stream));
-        for (uint32_t it = 2; it < 8; ++it)
-            QSM_TRY(launch_variant(ctx, ctx->stream, k, v->tgv, false, v->tl[k].nact, pd_volume_args(*v, k, it),
-                                   v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it)));
-        QSM_CUDA(cudaEventRecord(t1, ctx->stream));
-        QSM_CUDA(cudaEventSynchronize(t1));
+                                   v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it), it > 0));
+        // six iterations, then, where those take under 0.3 ms, 36 more
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, t0, t1);
+        for (uint32_t i0 = 2, n = 6;; n = 36) {
+            QSM_CUDA(cudaEventRecord(t0, ctx->stream));
+            for (uint32_t it = i0; it < i0 + n; ++it)
+                QSM_TRY(launch_variant(ctx, ctx->stream, k, v->tgv, false, v->tl[k].nact, pd_volume_args(*v, k, it),
+                                       v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it), true));
+            QSM_CUDA(cudaEventRecord(t1, ctx->stream));
+            QSM_CUDA(cudaEventSynchronize(t1));
+            cudaEventElapsedTime(&ms, t0, t1);
+            ms /= (float)n;
+            i0 += n;
+            if (n != 6 || 6 * ms >= 0.3f) break;
+        }
         if (ms < best) {
             best = ms;
             v->var = k;
@@ -547,7 +567,7 @@ qsm_status pd_fused(qsm_ctx *ctx, bool tgv, const Dims &d, qsm_dtype dt, const v
         const bool chk = ((it + 1) % 10) == 0;
         if (!empty)
             QSM_TRY(launch_variant(ctx, ctx->stream, var, tgv, chk, nact, pd_volume_args(v, var, it), v.dc, v.pc, d,
-                                   tol, it + 1, volume_maps(v, var, it)));
+                                   tol, it + 1, volume_maps(v, var, it), it > 0));
         enq = it + 1;
         const bool print = verbose && (it == 0 || it == maxiter - 1 || ((it + 1) % pmod) == 0);
         if (print || (chk && ((it + 1) % 100) == 0)) {

@@ -13,11 +13,13 @@ __global__ void __launch_bounds__((TX + 4) * (TY + 4), TGV ? 1 : 2)
 stream_k(FusedArgs s, DualC<float> dc, PrimalC<float> pc, Dims d, int cz, double tol, uint32_t it)
 {
     extern __shared__ double smem_raw[];
+    const unsigned tile = __ldg(s.tiles + blockIdx.x);
+    pdl_begin();
     if (s.ctl->done) return;
     const uint32_t itn = launch_iter(s, it);
     if (!itn) return;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    column_pd<TX, TY, TGV>(s, dc, pc, d, cz, s.tiles[blockIdx.x], CHECK, (float *)smem_raw, acc);
+    column_pd<TX, TY, TGV>(s, dc, pc, d, cz, tile, CHECK, (float *)smem_raw, acc);
     if (CHECK) monitor_reduce<(TX + 4) * (TY + 4)>(s, smem_raw, acc, tol, itn);
 }
 
@@ -27,12 +29,14 @@ stream_tma_k(const __grid_constant__ TmaMaps tm, FusedArgs s, DualC<float> dc, P
              double tol, uint32_t it)
 {
     extern __shared__ __align__(16) unsigned char smem_tma[];
+    const unsigned tile = __ldg(s.tiles + blockIdx.x);
+    pdl_begin();
     if (s.ctl->done) return;
     const uint32_t itn = launch_iter(s, it);
     if (!itn) return;
     char *base = tma_smem_base(smem_tma);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    column_tma<TX, TY>(tm, s, dc, pc, d, cz, s.tiles[blockIdx.x], CHECK, base, acc);
+    column_tma<TX, TY>(tm, s, dc, pc, d, cz, tile, CHECK, base, acc);
     // the monitor fold reuses shared memory past the plane barriers
     if (CHECK) monitor_reduce<(TX + 4) * (TY + 4)>(s, (double *)(base + 128), acc, tol, itn);
 }
@@ -86,46 +90,46 @@ qsm_status stream_set_smem(qsm_ctx *ctx)
 }
 
 template <int TX, int TY>
-static void launch_tma_t(cudaStream_t st, bool chk, unsigned nact, const TmaMaps &tm, const FusedArgs &s,
+static void launch_tma_t(cudaStream_t st, bool chain, bool chk, unsigned nact, const TmaMaps &tm, const FusedArgs &s,
                          const DualC<float> &dc, const PrimalC<float> &pc, const Dims &d, int cz, double tol,
                          uint32_t it)
 {
     const size_t sm = TmaLayout<TX, TY>::REQUEST;
     const int nt = (TX + 4) * (TY + 4);
-    if (chk) stream_tma_k<TX, TY, true><<<nact, nt, sm, st>>>(tm, s, dc, pc, d, cz, tol, it);
-    else stream_tma_k<TX, TY, false><<<nact, nt, sm, st>>>(tm, s, dc, pc, d, cz, tol, it);
+    launch_iteration(chk ? stream_tma_k<TX, TY, true> : stream_tma_k<TX, TY, false>, chain, nact, nt, sm, st, tm, s, dc, pc, d,
+                     cz, tol, it);
 }
 
 template <int TX, int TY>
-static void launch_t(cudaStream_t st, bool tgv, bool chk, unsigned nact, const FusedArgs &s, const DualC<float> &dc,
+static void launch_t(cudaStream_t st, bool chain, bool tgv, bool chk, unsigned nact, const FusedArgs &s, const DualC<float> &dc,
                      const PrimalC<float> &pc, const Dims &d, int cz, double tol, uint32_t it)
 {
     const size_t sm = stream_smem(TX, TY, tgv);
     const int nt = (TX + 4) * (TY + 4);
     if (tgv) {
-        if (chk) stream_k<TX, TY, true, true><<<nact, nt, sm, st>>>(s, dc, pc, d, cz, tol, it);
-        else stream_k<TX, TY, true, false><<<nact, nt, sm, st>>>(s, dc, pc, d, cz, tol, it);
+        launch_iteration(chk ? stream_k<TX, TY, true, true> : stream_k<TX, TY, true, false>, chain, nact, nt, sm, st, s, dc, pc, d,
+                         cz, tol, it);
     } else {
-        if (chk) stream_k<TX, TY, false, true><<<nact, nt, sm, st>>>(s, dc, pc, d, cz, tol, it);
-        else stream_k<TX, TY, false, false><<<nact, nt, sm, st>>>(s, dc, pc, d, cz, tol, it);
+        launch_iteration(chk ? stream_k<TX, TY, false, true> : stream_k<TX, TY, false, false>, chain, nact, nt, sm, st, s, dc, pc,
+                         d, cz, tol, it);
     }
 }
 
 qsm_status stream_launch(qsm_ctx *ctx, cudaStream_t st, int tx, int ty, int cz, bool tgv, bool chk, unsigned nact,
                          const FusedArgs &s, const DualC<float> &dc, const PrimalC<float> &pc, const Dims &d,
-                         double tol, uint32_t it, const TmaMaps *tm)
+                         double tol, uint32_t it, const TmaMaps *tm, bool chain)
 {
     if (tm) {
         if (!tgv) return QSM_ERR_ARG;
-        if (tx == 28 && ty == 16) launch_tma_t<28, 16>(st, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
-        else if (tx == 28 && ty == 20) launch_tma_t<28, 20>(st, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
-        else if (tx == 28 && ty == 24) launch_tma_t<28, 24>(st, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
+        if (tx == 28 && ty == 16) launch_tma_t<28, 16>(st, chain, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
+        else if (tx == 28 && ty == 20) launch_tma_t<28, 20>(st, chain, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
+        else if (tx == 28 && ty == 24) launch_tma_t<28, 24>(st, chain, chk, nact, *tm, s, dc, pc, d, cz, tol, it);
         else return QSM_ERR_ARG;
         QSM_CUDA(cudaGetLastError());
         return QSM_OK;
     }
-    if (tx == 28 && ty == 12) launch_t<28, 12>(st, tgv, chk, nact, s, dc, pc, d, cz, tol, it);
-    else if (tx == 28 && ty == 16) launch_t<28, 16>(st, tgv, chk, nact, s, dc, pc, d, cz, tol, it);
+    if (tx == 28 && ty == 12) launch_t<28, 12>(st, chain, tgv, chk, nact, s, dc, pc, d, cz, tol, it);
+    else if (tx == 28 && ty == 16) launch_t<28, 16>(st, chain, tgv, chk, nact, s, dc, pc, d, cz, tol, it);
     else return QSM_ERR_ARG;
     QSM_CUDA(cudaGetLastError());
     return QSM_OK;
