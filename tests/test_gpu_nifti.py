@@ -131,3 +131,62 @@ def test_fortran_ordered_tensor_saves_in_matlab_order(qn, nio, tmp_path):
         assert open(tmp_path / name, "rb").read() == nio.save_bytes(chi, [1, 1, 1])
     with pytest.raises(ValueError, match="contiguous"):
         qn.header_bytes(torch.zeros((6, 6, 6), device="cuda")[:, ::2, :])
+
+
+@pytest.mark.parametrize("dt", [2, 256, 4, 512, 16])
+@pytest.mark.parametrize("slope,inter", [(0.1, 0.0), (0.1, -0.3), (1.0, 0.0), (1.0, 16777216.0), (2.0, 16777217.0), (0.25, -3.0),
+                                         (3e-4, 1234.5), (-7.7, 1e-5), (1.0, -100.0), (1e-30, 1.0), (2.0 ** -24, 1.0),
+                                         (3 * 2.0 ** -25, 1.0), (1e25, -1e12)])
+def test_scaling_in_singles_bitexact(qn, nio, dt, slope, inter):
+    """Scaled 8- and 16-bit and single images: every stored value (singles: also
+    zeros of both signs, subnormals, huge values, infinities, NaN), with factors
+    whose sums are exact, fall midway between two singles, cancel, or leave the
+    range the single arithmetic takes.  Bit for bit against load_nii's formula,
+    single(slope * double(x) + inter)."""
+    t = np.dtype(nio.DT[dt])
+    if t.kind == "f":
+        rng = np.random.default_rng(3)
+        x = (rng.standard_normal(65536) * 10.0 ** rng.uniform(-45, 38, 65536)).astype(t)
+        x[:9] = [0.0, -0.0, 1e-45, -1e-38, 3e38, np.inf, -np.inf, np.nan, 1.0]
+        x[9:4000] = np.arange(9, 4000)
+    else:
+        x = np.arange(1 << (8 * t.itemsize)).astype(np.dtype("u%d" % t.itemsize)).view(t)
+    n = x.size
+    hb = build_header("<", datatype=dt, dim=(3, 32, n // 32, 1, 1, 1, 1, 1), slope=slope, inter=inter)
+    s32, i32 = np.float64(np.float32(slope)), np.float64(np.float32(inter))
+    with np.errstate(all="ignore"):
+        want = (s32 * x.astype(np.float64) + i32).astype(np.float32)
+    img, h = qn.decode(hb, x.tobytes())
+    if (slope, inter) == (1.0, 0.0):  # load_nii applies no such scaling: the stored class as it is
+        assert not h.scaled and img.dtype == t and img.tobytes(order="F") == x.tobytes()
+        return
+    assert h.scaled and img.dtype == np.float32
+    got = img.ravel(order="F")
+    nan = np.isnan(want)
+    assert np.array_equal(np.isnan(got), nan)
+    assert np.array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32))
+    wide = qn.decode(hb, x.tobytes(), out_dtype=np.float64)[0].ravel(order="F")
+    assert np.array_equal(wide[~nan], want[~nan].astype(np.float64))
+
+
+@pytest.mark.parametrize("dt", [2, 4, 16])
+@pytest.mark.parametrize("nx", [4, 8, 30, 33, 260])
+@pytest.mark.parametrize("sx", [1, -1])
+@pytest.mark.parametrize("endian", ["<", ">"])
+def test_scaling_quads(qn, nio, dt, nx, sx, endian):
+    """Rows of four-voxel quads (row length a multiple of four, running along the
+    stored rows in either direction) and rows that are none, from aligned device
+    buffers and ones that start inside a quad."""
+    torch = pytest.importorskip("torch")
+    kw = dict(datatype=dt, dim=(4, nx, 5, 3, 2, 1, 1, 1), slope=0.37, inter=-3.1, sform=1,
+              srow=[[sx, 0, 0, 0], [0, -1, 0, 0], [0, 0, 1, 0]])
+    hb = build_header(endian, **kw)
+    pl = _payload(nio, dt, nx * 30, endian, nx)
+    ref, _ = nio.load_nii(hb, pl)
+    esz = np.dtype(nio.DT[dt]).itemsize
+    for shift in (0, esz):
+        buf = torch.zeros(len(pl) + 64, dtype=torch.uint8, device="cuda")
+        buf[shift:shift + len(pl)] = torch.from_numpy(np.frombuffer(pl, np.uint8).copy()).cuda()
+        img, _ = qn.decode(hb, buf[shift:shift + len(pl)], device=True)
+        got = img.cpu().numpy().T
+        assert got.shape == ref.shape and np.array_equal(got, ref)
