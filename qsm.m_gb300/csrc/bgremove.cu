@@ -18,7 +18,6 @@
 // code evaluates them (single mask, so single FFTs); the field arithmetic is
 // in the class of f.  Reductions (iSMV residuals) accumulate in FP64 in a
 // fixed order.
-#include <cufft.h>
 #include <float.h>
 #include <math.h>
 #include <stdio.h>
@@ -27,6 +26,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft_plans.cuh"
 
 namespace qsm {
 
@@ -498,56 +498,33 @@ const char *fft_str(cufftResult r)
 // R2C / C2R plans of one padded grid, in T and in FP32 (eroded masks)
 template <typename T>
 struct Plans {
-    cufftHandle f = 0, i = 0, f32 = 0, i32 = 0;
-    bool hf = false, hi = false, hf32 = false, hi32 = false;
-    void destroy()
+    FftPlans p;
+    void destroy(qsm_ctx *ctx) { fft_release(ctx, &p); }
+    qsm_status make(qsm_ctx *ctx, const Dims &d)
     {
-        if (hf) cufftDestroy(f);
-        if (hi) cufftDestroy(i);
-        if (hf32) cufftDestroy(f32);
-        if (hi32) cufftDestroy(i32);
-        hf = hi = hf32 = hi32 = false;
-    }
-    qsm_status make(qsm_ctx *ctx, const Dims &p)
-    {
-        const int nx = (int)p.nx, ny = (int)p.ny, nz = (int)p.nz;
-        const bool dbl = sizeof(T) == 8;
-        BG_FFT(cufftPlan3d(&f, nz, ny, nx, dbl ? CUFFT_D2Z : CUFFT_R2C));
-        hf = true;
-        BG_FFT(cufftPlan3d(&i, nz, ny, nx, dbl ? CUFFT_Z2D : CUFFT_C2R));
-        hi = true;
-        BG_FFT(cufftSetStream(f, ctx->stream));
-        BG_FFT(cufftSetStream(i, ctx->stream));
-        if (dbl) {
-            BG_FFT(cufftPlan3d(&f32, nz, ny, nx, CUFFT_R2C));
-            hf32 = true;
-            BG_FFT(cufftPlan3d(&i32, nz, ny, nx, CUFFT_C2R));
-            hi32 = true;
-            BG_FFT(cufftSetStream(f32, ctx->stream));
-            BG_FFT(cufftSetStream(i32, ctx->stream));
-        }
-        return QSM_OK;
+        const cufftType f64[4] = {CUFFT_D2Z, CUFFT_Z2D, CUFFT_R2C, CUFFT_C2R}, f32[2] = {CUFFT_R2C, CUFFT_C2R};
+        return sizeof(T) == 8 ? fft_acquire(ctx, d, f64, 4, &p) : fft_acquire(ctx, d, f32, 2, &p);
     }
     qsm_status fwd(qsm_ctx *ctx, T *in, typename Cx<T>::type *out)
     {
-        if (sizeof(T) == 8) BG_FFT(cufftExecD2Z(f, (cufftDoubleReal *)in, (cufftDoubleComplex *)out));
-        else BG_FFT(cufftExecR2C(f, (cufftReal *)in, (cufftComplex *)out));
+        if (sizeof(T) == 8) BG_FFT(cufftExecD2Z(p.h[0], (cufftDoubleReal *)in, (cufftDoubleComplex *)out));
+        else BG_FFT(cufftExecR2C(p.h[0], (cufftReal *)in, (cufftComplex *)out));
         return QSM_OK;
     }
     qsm_status inv(qsm_ctx *ctx, typename Cx<T>::type *in, T *out)
     {
-        if (sizeof(T) == 8) BG_FFT(cufftExecZ2D(i, (cufftDoubleComplex *)in, (cufftDoubleReal *)out));
-        else BG_FFT(cufftExecC2R(i, (cufftComplex *)in, (cufftReal *)out));
+        if (sizeof(T) == 8) BG_FFT(cufftExecZ2D(p.h[1], (cufftDoubleComplex *)in, (cufftDoubleReal *)out));
+        else BG_FFT(cufftExecC2R(p.h[1], (cufftComplex *)in, (cufftReal *)out));
         return QSM_OK;
     }
     qsm_status fwd32(qsm_ctx *ctx, float *in, cufftComplex *out)
     {
-        BG_FFT(cufftExecR2C(sizeof(T) == 8 ? f32 : f, in, out));
+        BG_FFT(cufftExecR2C(p.h[sizeof(T) == 8 ? 2 : 0], in, out));
         return QSM_OK;
     }
     qsm_status inv32(qsm_ctx *ctx, cufftComplex *in, float *out)
     {
-        BG_FFT(cufftExecC2R(sizeof(T) == 8 ? i32 : i, in, out));
+        BG_FFT(cufftExecC2R(p.h[sizeof(T) == 8 ? 3 : 1], in, out));
         return QSM_OK;
     }
 };
@@ -739,14 +716,14 @@ qsm_status run(qsm_ctx *ctx, Method meth, const Dims &d, size_t ne, const T *f, 
     qsm_status st = pl.make(ctx, g.p);
     if (st == QSM_OK) st = w.alloc(ctx, g);
     if (st != QSM_OK) {
-        pl.destroy();
+        pl.destroy(ctx);
         w.release(ctx);
         return st;
     }
     const unsigned gn = grid_for(N), gh = grid_for(nh);
     T *kv = nullptr;  // RESHARP's eight Krylov vectors
     if (meth == RESHARP && (st = dalloc(ctx, (void **)&kv, 8 * N * sizeof(T))) != QSM_OK) {
-        pl.destroy();
+        pl.destroy(ctx);
         w.release(ctx);
         return st;
     }
@@ -922,7 +899,7 @@ qsm_status run(qsm_ctx *ctx, Method meth, const Dims &d, size_t ne, const T *f, 
     st = body();
     cudaStreamSynchronize(ctx->stream);
     if (kv) dfree(ctx, kv);
-    pl.destroy();
+    pl.destroy(ctx);
     w.release(ctx);
     return st;
 }
@@ -1054,7 +1031,7 @@ qsm_status run_pdf(qsm_ctx *ctx, const Dims &d, size_t ne, const T *f, const uin
     void *blk = nullptr;
     qsm_status st = dalloc(ctx, &blk, 8 * rb + 2 * cb + (BG_GRID + 64) * sizeof(double));
     if (st != QSM_OK) {
-        pl.destroy();
+        pl.destroy(ctx);
         return st;
     }
     char *p = (char *)blk;
@@ -1218,7 +1195,7 @@ qsm_status run_pdf(qsm_ctx *ctx, const Dims &d, size_t ne, const T *f, const uin
     };
     st = body();
     cudaStreamSynchronize(ctx->stream);
-    pl.destroy();
+    pl.destroy(ctx);
     dfree(ctx, blk);
     return st;
 }

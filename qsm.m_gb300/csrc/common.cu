@@ -3,6 +3,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "fft_plans.cuh"
 #include "fp64.cuh"
 
 namespace qsm {
@@ -361,6 +362,7 @@ qsm_status qsm_ctx_destroy(qsm_ctx *ctx)
     if (!ctx) return QSM_OK;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    fft_clear(ctx);
     if (ctx->red_partial) cudaFree(ctx->red_partial);
     if (ctx->red_out) cudaFree(ctx->red_out);
     if (ctx->red_count) cudaFree(ctx->red_count);

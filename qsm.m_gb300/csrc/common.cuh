@@ -95,6 +95,8 @@ static inline dim3 vox_grid(const Dims &d)
 // context
 // ---------------------------------------------------------------------------
 
+struct FftCache;  // cuFFT plans kept between calls (fft_plans.cu)
+
 }  // namespace qsm
 
 struct qsm_ctx {
@@ -110,6 +112,7 @@ struct qsm_ctx {
     unsigned int *red_count;
     double *host_out;      // pinned, 8 doubles
     uint32_t debug;        // QSM_DEBUG_* test hooks (qsm_ctx_set_debug)
+    qsm::FftCache *fft;    // null until the first transform
 };
 
 namespace qsm {

@@ -26,13 +26,13 @@
 // FP64 (the MATLAB default class) or FP32 arithmetic by dtype; every
 // reduction accumulates in FP64 with a fixed order (block partials folded
 // in block order), so results are run-to-run deterministic.
-#include <cufft.h>
 #include <math.h>
 #include <stdio.h>
 
 #include <algorithm>
 
 #include "common.cuh"
+#include "fft_plans.cuh"
 
 namespace qsm {
 
@@ -555,9 +555,8 @@ static qsm_status tv_run(qsm_ctx *ctx, const Dims &d, const S *f, const uint8_t 
     double *ctl = sums + 64;
 
     qsm_status st = QSM_OK;
-    cufftHandle pf = 0, pi = 0;
-    bool havef = false, havei = false;
-    const cufftType tf = sizeof(T) == 8 ? CUFFT_D2Z : CUFFT_R2C, ti = sizeof(T) == 8 ? CUFFT_Z2D : CUFFT_C2R;
+    FftPlans plans;  // forward, inverse
+    const cufftType types[2] = {sizeof(T) == 8 ? CUFFT_D2Z : CUFFT_R2C, sizeof(T) == 8 ? CUFFT_Z2D : CUFFT_C2R};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     double hc[C_N] = {};
     int cur = 0;
@@ -579,12 +578,7 @@ static qsm_status tv_run(qsm_ctx *ctx, const Dims &d, const S *f, const uint8_t 
     const unsigned gk = (unsigned)std::min<size_t>((nh + TV_BLOCK - 1) / TV_BLOCK, (size_t)TV_GRID);
 
     QSM_STEP(cuda_st(ctx, cudaMemsetAsync(lmb[0], 0, 3 * N * sizeof(T), ctx->stream), "memset"));
-    QSM_FFT(cufftPlan3d(&pf, (int)d.nz, (int)d.ny, (int)d.nx, tf));
-    havef = true;
-    QSM_FFT(cufftPlan3d(&pi, (int)d.nz, (int)d.ny, (int)d.nx, ti));
-    havei = true;
-    QSM_FFT(cufftSetStream(pf, ctx->stream));
-    QSM_FFT(cufftSetStream(pi, ctx->stream));
+    QSM_STEP(fft_acquire(ctx, d, types, 2, &plans));
     QSM_STEP(cuda_st(ctx, cudaEventCreate(&e0), "event"));
     QSM_STEP(cuda_st(ctx, cudaEventCreate(&e1), "event"));
     QSM_STEP(cuda_st(ctx, cudaEventRecord(e0, ctx->stream), "event"));
@@ -594,8 +588,8 @@ static qsm_status tv_run(qsm_ctx *ctx, const Dims &d, const S *f, const uint8_t 
     dq_k<T><<<gk, TV_BLOCK, 0, ctx->stream>>>(Dq, tab, K);
     // u = f; fhat = fft3(f) (F = mu conj(D) fhat is formed in kmul_k)
     cvt_in_k<T, S><<<g, b, 0, ctx->stream>>>(u, f, N);
-    if (sizeof(T) == 8) QSM_FFT(cufftExecD2Z(pf, (cufftDoubleReal *)u, (cufftDoubleComplex *)fhat));
-    else QSM_FFT(cufftExecR2C(pf, (cufftReal *)u, (cufftComplex *)fhat));
+    if (sizeof(T) == 8) QSM_FFT(cufftExecD2Z(plans.h[0], (cufftDoubleReal *)u, (cufftDoubleComplex *)fhat));
+    else QSM_FFT(cufftExecR2C(plans.h[0], (cufftReal *)u, (cufftComplex *)fhat));
     grad_init_k<T><<<g, b, 0, ctx->stream>>>(v[0], u, d, ihx, ihy, ihz, part);
     fold_k<<<1, TV_BLOCK, 0, ctx->stream>>>(sums, part, 1, TV_GRID, 0, 0);
     // control state: rho, 1/rho (as the host forms it), nr of the initial v, flag 0
@@ -621,11 +615,11 @@ static qsm_status tv_run(qsm_ctx *ctx, const Dims &d, const S *f, const uint8_t 
                 const int nxt = cur ^ 1;
                 // u-subproblem
                 adj_rhs_k<T><<<g, b, 0, ctx->stream>>>(r, v[cur], lmb[lc], d, -ihx, -ihy, -ihz, ctl, ii, usave, u);
-                if (sizeof(T) == 8) QSM_FFT(cufftExecD2Z(pf, (cufftDoubleReal *)r, (cufftDoubleComplex *)R));
-                else QSM_FFT(cufftExecR2C(pf, (cufftReal *)r, (cufftComplex *)R));
+                if (sizeof(T) == 8) QSM_FFT(cufftExecD2Z(plans.h[0], (cufftDoubleReal *)r, (cufftDoubleComplex *)R));
+                else QSM_FFT(cufftExecR2C(plans.h[0], (cufftReal *)r, (cufftComplex *)R));
                 kmul_k<T><<<gk, TV_BLOCK, 0, ctx->stream>>>(R, fhat, Dq, tab, K, ctl, 1.0 / (double)N);
-                if (sizeof(T) == 8) QSM_FFT(cufftExecZ2D(pi, (cufftDoubleComplex *)R, (cufftDoubleReal *)u));
-                else QSM_FFT(cufftExecC2R(pi, (cufftComplex *)R, (cufftReal *)u));
+                if (sizeof(T) == 8) QSM_FFT(cufftExecZ2D(plans.h[1], (cufftDoubleComplex *)R, (cufftDoubleReal *)u));
+                else QSM_FFT(cufftExecC2R(plans.h[1], (cufftComplex *)R, (cufftReal *)u));
                 // v-subproblem, multipliers, residuals
                 if (sizeof(T) == 4 && o.tv == 1) {
                     grad_shrink_norms_k<T><<<gs, b, 0, ctx->stream>>>(v[nxt], v[cur], lmb[lc ^ 1], lmb[lc], u, d, ihx,
@@ -678,8 +672,7 @@ static qsm_status tv_run(qsm_ctx *ctx, const Dims &d, const S *f, const uint8_t 
 done:
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    if (havef) cufftDestroy(pf);
-    if (havei) cufftDestroy(pi);
+    fft_release(ctx, &plans);
     qsm_status st2 = dfree(ctx, blk);
     return st != QSM_OK ? st : st2;
 }

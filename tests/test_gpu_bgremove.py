@@ -176,3 +176,25 @@ def test_pdf_errors(gpu_ctx, qsm):
         qsm.pdf(f, m, [1, 0, 1])
     with pytest.raises(ValueError):
         qsm.pdf(f, m, [1, 1, 1], w=np.ones((5, 5, 5)))
+
+
+def test_kept_plans(gpu_ctx, qsm, bg):
+    """Transforms with plans made earlier, in one context: more sizes and types
+    than a context keeps (12 plans; a double field takes four), so the second
+    pass meets kept, dropped and remade plans.  Equal to the bit with the first
+    pass; FP64 within the oracle's bound."""
+    shapes = [(24, 22, 20), (20, 22, 24), (23, 21, 26), (26, 24, 22), (22, 20, 24)]
+    first = {}
+    for turn in range(2):
+        for k, shape in enumerate(shapes if turn == 0 else shapes[::-1]):
+            for dt in (np.float64, np.float32):
+                f, m = _case(shape, 40 + shape[0])
+                fl, mo = qsm.sharp(f.astype(dt), m, [1, 1, 1], 3.0, 0.05)
+                if turn == 0:
+                    first[shape, dt] = fl
+                    if dt is np.float64:
+                        rfl, rmo = bg.sharp(f, m, [1, 1, 1], 3.0, 0.05)
+                        assert np.array_equal(mo, rmo)
+                        assert _rel(fl, rfl) <= 1e-9
+                else:
+                    assert np.array_equal(fl, first[shape, dt])
