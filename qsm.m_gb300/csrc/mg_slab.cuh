@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     uint32_t *exp[2] = {(uint32_t *)(smraw + lay.exp[0]), (uint32_t *)(smraw + lay.exp[1])};
     uint8_t *need = smraw + lay.need;  // [colour][slot]: a received value some voxel of the chunk reads
     const uint32_t *list[2] = {l0, l1};
-    for (int t = tid; t < 2 * ((int)cn + 1); t += blockDim.x) bnd[t] = tab.cut[2 * (t / 2 * (SL_MAX_CTAS / (int)cn)) + t % 2];
+    chain_early();
     if (tid < 2) {
         nexp[tid] = 0;
         nrecv[tid] = 0;
@@ -294,6 +294,8 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     for (unsigned t = tid; t < 2 * len; t += blockDim.x) v[0][t] = (T)0;  // both colours: the arrays are adjacent
     if (cn > 1)
         for (unsigned t = tid; t < 2 * len; t += blockDim.x) need[t] = 0;
+    chain_wait();
+    for (int t = tid; t < 2 * ((int)cn + 1); t += blockDim.x) bnd[t] = tab.cut[2 * (t / 2 * (SL_MAX_CTAS / (int)cn)) + t % 2];
     __syncthreads();
     const unsigned start[2] = {bnd[2 * c], bnd[2 * c + 1]};
     const unsigned cnt[2] = {bnd[2 * c + 2] - start[0], bnd[2 * c + 3] - start[1]};

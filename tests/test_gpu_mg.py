@@ -455,3 +455,24 @@ def test_coarse_packets_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl, kind):
     a = qsm.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl, info=gi)
     assert gi["coarse_ctas"] < 0
     assert bits_equal(a, port.mg_mex(v0, f, m, h, -1.0, 1, 1, 2, 2, 2, nl))
+
+
+@pytest.mark.parametrize("dt", ("float64", "float32"))
+@pytest.mark.parametrize("shape,nl", [((64, 60, 52), 3), ((63, 41, 30), 4)])
+def test_cycles_reuse_levels_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl):
+    """Levels a cycle finds as an earlier one left them: v cleared on the voxel
+    lists alone, the whole-GPU sweeps' barrier count run on.  Several cycles,
+    W-cycles (two visits of a level between clearings) and FMG, whose prolongation
+    writes a level's v in between: to the bit the oracle's."""
+    import qsm_gb300.synthetic as S
+
+    f, m, _ = S.poisson_case(shape, 21, semi=(0.3 * shape[2], 0.46 * shape[0]))
+    f = np.asfortranarray(f.astype(dt))
+    v0 = np.zeros(shape, dt, order="F")
+    for mu in (1, 2):
+        b = port.mg_mex(v0, f, m, [1, 1, 1], -1.0, 3, mu, 2, 1, 2, nl)
+        a = qsm.mg_mex(v0, f, m, [1, 1, 1], -1.0, 3, mu, 2, 1, 2, nl)
+        assert bits_equal(a, b), first_diff(a, b)
+        b = port.fmg_mex(f, m, [1, 1, 1], -1.0, 2, mu, 1, 2, 2, nl)
+        a = qsm.fmg_mex(f, m, [1, 1, 1], -1.0, 2, mu, 1, 2, 2, nl)
+        assert bits_equal(a, b), first_diff(a, b)
