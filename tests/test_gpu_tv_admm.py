@@ -110,3 +110,22 @@ def test_tv_errors(gpu_ctx, qsm):
         qsm.tv(np.zeros((8, 8, 2)), np.ones((8, 8, 2), np.uint8), [1, 1, 1])
     with pytest.raises(qsm.QsmError, match="ARG"):
         qsm.tv(np.zeros((8, 8, 8)), np.ones((8, 8, 8), np.uint8), [1, 1, 1], opts=dict(tv=3))
+
+
+@pytest.mark.parametrize("shape", [(33, 5, 40), (64, 9, 7), (31, 4, 3), (3, 70, 12), (97, 33, 66)])
+def test_tv_tile_edges(gpu_ctx, qsm, tvo, shape):
+    """Tiles of 32 columns and a few rows, chunks of planes, several tiles a block:
+    a column, row or plane beyond a tile, short tiles, the smallest sizes, every neighbour
+    periodic.  A field of noise without a mask, so that every edge counts; the bounds
+    of the tests above (FP64 1e-9, FP32 1e-4), for the residual sums as well."""
+    rng = np.random.default_rng(sum(shape))
+    f = np.asfortranarray(rng.normal(0.0, 0.05, shape))
+    m = np.ones(shape, np.uint8, order="F")
+    opts = dict(maxit=5, tv=1, rtol=0.0, atol=0.0)
+    trace, info = [], {}
+    ref = tvo.tv(f, m, [1, 0.8, 1.3], opts=opts, trace=trace)
+    for dt, tol in ((np.float64, 1e-9), (np.float32, 1e-4)):
+        x = qsm.tv(f.astype(dt), m, [1, 0.8, 1.3], opts=opts, info=info)
+        assert _rel(x, ref) <= tol, first_diff(x, ref.astype(dt))
+        assert abs(info["nr"] - trace[-1]["nr"]) <= tol * trace[-1]["nr"]
+        assert abs(info["ns"] - trace[-1]["ns"]) <= tol * trace[-1]["ns"]
