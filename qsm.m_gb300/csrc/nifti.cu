@@ -234,31 +234,34 @@ __global__ void __launch_bounds__(256) convert_k(O *__restrict__ out, const S *_
     }
 }
 
-// single(slope * double(x) + inter) of an integer x of up to 16 bits or a single,
-// slope and inter singles (the product is then exact in FP64), without FP64: the exact sum as t + c + ce in singles (the
-// product's error by fused multiply-add, Knuth's sums), r the nearest single of t +
-// c and d what is left.  r is the result unless d + ce is within 2^-16 of half a
-// unit of r (or r is a power of two, whose lower neighbour is nearer): only there
-// could the rounding to double, or ce, decide, and *sure is false.
+// single(slope * double(x) + inter) of an integer x of up to 16 bits or a single
+// (INT: an integer), slope and inter singles (the product is then exact in FP64),
+// without FP64: y, one fused multiply-add, is the exact value v's nearest single.
+// Rounding to double first can only decide otherwise where v lies within 2^-28 of
+// half a unit of y, so *sure is false from 2^-15 on.  v - y comes in singles from
+// the product and its error (pe, exact by fused multiply-add) and Knuth's sum t +
+// te of the product and inter: t - y is exact (both are multiples of y's or t's
+// unit and differ by less than 2^24 of it), the two sums after it round by 2^-24.
 __device__ __forceinline__ float two_sum(float a, float b, float *err)
 {
     const float t = a + b, z = t - a;
     *err = (a - (t - z)) + (b - z);
     return t;
 }
+template <bool INT>
 __device__ __forceinline__ float scale_single(float x, float slope, float inter, bool *sure)
 {
-    const float p = x * slope, pe = fmaf(x, slope, -p);
-    float te, ce, d;
-    const float t = two_sum(p, inter, &te), c = two_sum(te, pe, &ce), r = two_sum(t, c, &d);
-    const uint32_t u = __float_as_uint(r) & 0x7fffffffu;
-    const bool exact = d == 0.0f && ce == 0.0f;
-    // half a unit in r's last place: 2^(e - 24)
-    const float half = __uint_as_float((u & 0x7f800000u) - (24u << 23));
+    const float p = x * slope, pe = fmaf(x, slope, -p), y = fmaf(x, slope, inter);
+    float te;
+    const float t = two_sum(p, inter, &te), e = ((t - y) + te) + pe;
+    // half a unit on y's lower side (that of the single before y: a power of two has the
+    // nearer neighbour there); y = 0 is exact
+    const uint32_t u = __float_as_uint(y) & 0x7fffffffu;
+    const float half = __uint_as_float(((u - 1u) & 0x7f800000u) - (24u << 23));
+    *sure = fabsf(e) * (1.0f + 1.0f / 32768.0f) < half;
     // (outside this range of a stored single the error terms might underflow or overflow)
-    const bool mid = x == 0.0f || (fabsf(x) >= 0x1p-40f && fabsf(x) <= 0x1p60f);
-    *sure = mid && (exact || ((u & 0x7fffffu) != 0u && fabsf(d) + fabsf(ce) < half * (1.0f - 1.0f / 65536.0f)));
-    return r == 0.0f ? t : r;  // (t has the sign of an exact zero)
+    if (!INT) *sure = *sure && (x == 0.0f || (fabsf(x) >= 0x1p-40f && fabsf(x) <= 0x1p60f));
+    return y;
 }
 
 // (out of line: inlined it is predicated, and an FP64 instruction takes its slot in
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(256) scale_single_k(O *__restrict__ out, const
                 S v;
                 memcpy(&v, &w[q], sizeof(S));
                 bool sure;
-                float y = scale_single((float)v, slope, inter, &sure);
+                float y = scale_single<(S)0.5 == (S)0>((float)v, slope, inter, &sure);
                 if (!sure) y = scale_double((float)v, slope, inter);
                 if constexpr (sizeof(O) == 8) dst[x] = f32_to_f64(y);
                 else dst[x] = y;
@@ -311,35 +314,86 @@ __global__ void __launch_bounds__(256) scale_single_k(O *__restrict__ out, const
 
 // The same for rows that run along the stored rows, of a length, and at addresses,
 // that are multiples of four voxels: a thread takes four neighbours with one load
-// and one store.  nq = quads of a row, total quads below 2^32.
-template <typename S>
-__global__ void __launch_bounds__(256) scale_quads_k(float *__restrict__ out, const S *__restrict__ in, Orient o, float slope,
-                                                     float inter, uint32_t nq, uint32_t quads)
+// and one store, and its quads' places by carries from one to the next (the
+// divisions of row_map and its selects cost more than the four voxels: with them,
+// and 40 instructions a voxel in scale_single, a 154 MB pass took 82 us, bound by
+// issue; 36.5 us now).
+struct QuadWalk {
+    int64_t c0, a1, a2, a3;   // stored index of loaded (x, o1, o2, t): c0 + x (- x - 3 backwards) + a1 o1 + a2 o2 + a3 t
+    uint32_t nq, n1, n2;      // quads of a row, rows, planes
+    uint32_t quads;           // in all (below 2^32 less a grid's stride)
+    int back;
+};
+
+static QuadWalk quad_walk(const Orient &o)
+{
+    const int64_t st[3] = {1, o.m[0], o.m[0] * o.m[1]};
+    QuadWalk w;
+    w.back = o.flip[0];
+    w.c0 = o.flip[0] ? o.m[0] - 4 : 0;  // (perm[0] = 0)
+    int64_t a[3] = {0, 0, 0};
+    for (int j = 1; j < 3; ++j) {
+        const int s = o.perm[j];
+        a[j] = o.flip[j] ? -st[s] : st[s];
+        if (o.flip[j]) w.c0 += st[s] * (o.m[s] - 1);
+    }
+    w.a1 = a[1];
+    w.a2 = a[2];
+    w.a3 = o.m[0] * o.m[1] * o.m[2];
+    w.nq = (uint32_t)(o.n[0] / 4);
+    w.n1 = (uint32_t)o.n[1];
+    w.n2 = (uint32_t)o.n[2];
+    w.quads = (uint32_t)(o.total / 4);
+    return w;
+}
+
+template <typename S, bool SWAP>
+__global__ void __launch_bounds__(256) scale_quads_k(float *__restrict__ out, const S *__restrict__ in, QuadWalk w, float slope,
+                                                     float inter)
 {
     struct alignas(4 * sizeof(S)) Quad {
         typename Word<sizeof(S)>::T w[4];
     };
-    for (uint32_t t = blockIdx.x * 256 + threadIdx.x; t < quads; t += gridDim.x * 256) {
-        const uint32_t r = t / nq, x = 4 * (t - r * nq);
-        const RowMap rm = row_map(o, (int64_t)r);
-        const bool back = rm.step < 0;  // voxels x .. x + 3 are stored at base - x - 3 .. base - x
-        const Quad v = *reinterpret_cast<const Quad *>(in + (back ? rm.base - x - 3 : rm.base + x));
+    auto split = [&](uint32_t t, uint32_t &q, uint32_t &o1, uint32_t &o2, uint32_t &o3) {
+        const uint32_t r = t / w.nq, k = r / w.n1;
+        q = t - r * w.nq;
+        o1 = r - k * w.n1;
+        o3 = k / w.n2;
+        o2 = k - o3 * w.n2;
+    };
+    const uint32_t step = gridDim.x * 256;
+    uint32_t t = blockIdx.x * 256 + threadIdx.x, q, o1, o2, o3, dq, d1, d2, d3;
+    split(t, q, o1, o2, o3);
+    split(step, dq, d1, d2, d3);
+    for (; t < w.quads; t += step) {
+        const int64_t l = w.c0 + w.a1 * o1 + w.a2 * o2 + w.a3 * o3 + (w.back ? -4 * (int64_t)q : 4 * (int64_t)q);
+        const Quad v = *reinterpret_cast<const Quad *>(in + l);
         float e[4], y[4];
         bool all = true;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            typename Word<sizeof(S)>::T w = back ? v.w[3 - q] : v.w[q];
-            if (o.swap) w = Word<sizeof(S)>::bswap(w);
+        for (int k = 0; k < 4; ++k) {
+            typename Word<sizeof(S)>::T b = w.back ? v.w[3 - k] : v.w[k];
+            if (SWAP) b = Word<sizeof(S)>::bswap(b);
             S c;
-            memcpy(&c, &w, sizeof(S));
-            e[q] = (float)c;
+            memcpy(&c, &b, sizeof(S));
+            e[k] = (float)c;
             bool sure;
-            y[q] = scale_single(e[q], slope, inter, &sure);
+            y[k] = scale_single<(S)0.5 == (S)0>(e[k], slope, inter, &sure);
             all = all && sure;
         }
         float4 res = make_float4(y[0], y[1], y[2], y[3]);
         if (!all) res = scale_quad_double(make_float4(e[0], e[1], e[2], e[3]), slope, inter);  // (all four: the same bits)
         *reinterpret_cast<float4 *>(out + 4 * (size_t)t) = res;
+        q += dq;
+        uint32_t c = q >= w.nq;
+        q -= c ? w.nq : 0;
+        o1 += d1 + c;
+        c = o1 >= w.n1;
+        o1 -= c ? w.n1 : 0;
+        o2 += d2 + c;
+        c = o2 >= w.n2;
+        o2 -= c ? w.n2 : 0;
+        o3 += d3 + c;
     }
 }
 
@@ -689,17 +743,18 @@ qsm_status qsm_nifti_decode(qsm_ctx *ctx, const qsm_nifti_hdr *h, const void *pa
             break;
         }
     } else if (h->scaled && (eb <= 2 || sdt == 16) && to_single && single_factors(h->scl_slope, h->scl_inter)) {
-        // a 224 x 224 x 128 x 4 int16 series (154 MB): the whole call 122-126 us, against 158
+        // a 224 x 224 x 128 x 4 int16 series (154 MB): the whole call 75 us, against 158
         // through the table, whose gathers cost an L1 access per voxel; single 224 x 224 x 128 x 2:
-        // 81 against 144 us in FP64 (the four-voxel form; one by one 143 and 93 us)
+        // at most 81 against 144 us in FP64 (the four-voxel form; one by one 143 and 93 us)
         const int64_t quads = o.total / 4;
         const bool by4 = out_datatype != 64 && o.perm[0] == 0 && o.n[0] % 4 == 0 && quads < 0xffffffffll - 152 * 4096 &&
                          o.rows <= 0x7fffffff && (uintptr_t)in % (4 * eb) == 0 && (uintptr_t)so.dev % 16 == 0;
         const unsigned gq = (unsigned)std::min<int64_t>((quads + 255) / 256, 152 * 16);
+        const QuadWalk qw = by4 ? quad_walk(o) : QuadWalk{};
 #define QSM_SCALE(S)                                                                                             \
     if (by4)                                                                                                     \
-        scale_quads_k<S><<<gq, 256, 0, ctx->stream>>>((float *)so.dev, (const S *)in, o, (float)h->scl_slope,    \
-                                                      (float)h->scl_inter, (uint32_t)(o.n[0] / 4), (uint32_t)quads); \
+        (o.swap ? scale_quads_k<S, true> : scale_quads_k<S, false>)<<<gq, 256, 0, ctx->stream>>>(                \
+            (float *)so.dev, (const S *)in, qw, (float)h->scl_slope, (float)h->scl_inter);                       \
     else if (out_datatype == 64)                                                                                      \
         scale_single_k<S, double><<<g, blk, 0, ctx->stream>>>((double *)so.dev, (const S *)in, o,                \
                                                               (float)h->scl_slope, (float)h->scl_inter);         \
