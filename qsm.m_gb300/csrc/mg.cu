@@ -629,6 +629,9 @@ enum { SW_LAUNCH = 0, SW_CLUSTER = 1, SW_GRID = 2 };
 // grid 3.1 us at 7.4k, 3.6 us at 31k, 8.6 us at 126k (a thread then walks
 // several entries one after another); launches 4.7 us at 31k, 7.8 us at 126k,
 // 11 us at 334k.  So the grid takes lists of up to about one entry per thread.
+// (Chained launches cost ~1.2 us less each: lines at 12k or 25k take 0.3 % off a 256^3 FP64
+// solve and add 0.1 % to LBV's; FP32 lists above 3k off the cluster take 4 % off 181 x 217
+// x 155 and add 1-3 % to 96^2 x 64 and 256^2 x 160.)
 constexpr unsigned SW_CLUSTER_MAX = 2500, SW_GRID_MAX = 45000;
 
 // A thread's share of one list: at most SW_PER entries (longer lists keep one
