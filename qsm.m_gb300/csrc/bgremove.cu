@@ -136,9 +136,13 @@ __global__ void smv_k(T *h, Dims pd, double hx, double hy, double hz, double r2,
 //   H(k) = 1/count sum_dz c(kz, dz) sum_dy c(ky, dy) C(kx, w(dy, dz)),
 //   c(k, 0) = 1, c(k, d) = 2 cos(2 pi k d / n), C(k, w) = sum_{d <= w} c(k, d):
 // ~R products per point and the tables, against a double transform of the whole
-// grid whose only nonzero points are the sphere's (202 x 202 x 120: 0.04 against
-// 1.2 ms with the points' test).  The sums run in pairs of doubles, so H carries the
-// tables' rounding alone, not that of partial sums up to the count.
+// grid whose only nonzero points are the sphere's (1.2 ms at 202 x 202 x 120 with the
+// points' test).  The sums run in 64-bit fixed point, each quantity scaled to its
+// bound: a product's high word is cut 2^-62 below the sum's bound, so H carries
+// the tables' rounding alone, not that of partial sums up to the count, and nothing
+// but the cosines and one conversion a point is FP64 (one pipe per SM; in pairs of
+// doubles the sums of one radius took 131 us at 210 x 210 x 126, the tables 33 and the
+// planes 14; now 12, 4.5 and 3).
 constexpr int SMV_MAX_R = 64;  // offsets per axis the direct sum takes
 struct SmvRows {
     int rz, ny[SMV_MAX_R];                  // dz = 0 .. rz; rows dy = 0 .. ny[dz] - 1
@@ -150,61 +154,76 @@ __device__ __forceinline__ double cos_term(size_t k, int d, size_t n)
     return d == 0 ? 1.0 : 2.0 * cospi(2.0 * (double)((k * (size_t)d) % n) / (double)n);
 }
 
-struct Pair {
-    double hi, lo;  // hi + lo
-    // + a b (Dekker's and Knuth's error terms; the products' by fused multiply-add)
-    __device__ __forceinline__ void add(double a, double b)
-    {
-        const double p = a * b, e = fma(a, b, -p), t = hi + p, z = t - hi;
-        lo += ((hi - (t - z)) + (p - z)) + e;
-        hi = t;
-    }
+struct SmvScale {
+    int cx, cy, cz, p, v;  // fixed-point fractions: C, the two factors, planes, sums
 };
 
-// cx[w nxh + kx] = C(kx, w); cy[d ny + ky], cz[d nz + kz] = c
-__global__ void smv_tables_k(double *cx, double *cy, double *cz, size_t nx, size_t nxh, size_t ny, size_t nz, int rx, int ry,
-                             int rz)
+static SmvScale smv_scale(int rx, int ry, int rz)
 {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nxh) {
-        Pair s{0.0, 0.0};
-        for (int d = 0; d <= rx; ++d) {
-            s.add(1.0, cos_term(t, d, nx));
-            cx[(size_t)d * nxh + t] = s.hi + s.lo;
+    auto bits = [](double v) { return (int)std::floor(std::log2(v)) + 1; };  // v < 2^bits
+    const double x = 2.0 * rx + 1.0, xy = x * (2.0 * ry + 1.0), xyz = xy * (2.0 * rz + 1.0);
+    SmvScale s;  // (a factor is at most 2: at most 61; a product's high word loses 64)
+    s.cx = 62 - bits(x);
+    s.p = std::min(62 - bits(xy), 61 + s.cx - 64);
+    s.cy = s.p + 64 - s.cx;
+    s.v = std::min(62 - bits(xyz), 61 + s.p - 64);
+    s.cz = s.v + 64 - s.p;
+    return s;
+}
+
+__device__ __forceinline__ long long fixed(double c, int scale)
+{
+    return __double2ll_rn(c * __longlong_as_double((long long)(1023 + scale) << 52));
+}
+
+// cx[w nxh + kx] = C(kx, w); cy[d ny + ky], cz[d nz + kz] = c; blockIdx.y: the axis
+__global__ void __launch_bounds__(256) smv_tables_k(long long *cx, long long *cy, long long *cz, size_t nx, size_t nxh, size_t ny,
+                                                    size_t nz, int rx, int ry, int rz, SmvScale S)
+{
+    __shared__ long long sh[SMV_MAX_R][32];
+    const size_t t = (size_t)blockIdx.x * 32 + threadIdx.x;
+    const int axis = (int)blockIdx.y;
+    const size_t n = axis == 0 ? nx : axis == 1 ? ny : nz, len = axis == 0 ? nxh : n;
+    const int r = axis == 0 ? rx : axis == 1 ? ry : rz, scale = axis == 0 ? S.cx : axis == 1 ? S.cy : S.cz;
+    long long *o = axis == 0 ? cx : axis == 1 ? cy : cz;
+    for (int d = (int)threadIdx.y; d <= r; d += 8)
+        if (t < len) {
+            const long long c = fixed(cos_term(t, d, n), scale);
+            if (axis == 0) sh[d][threadIdx.x] = c;
+            else o[(size_t)d * len + t] = c;
         }
-    }
-    if (t < ny)
-        for (int d = 0; d <= ry; ++d) cy[(size_t)d * ny + t] = cos_term(t, d, ny);
-    if (t < nz)
-        for (int d = 0; d <= rz; ++d) cz[(size_t)d * nz + t] = cos_term(t, d, nz);
+    if (axis != 0) return;  // (the block's)
+    __syncthreads();
+    for (int d = (int)threadIdx.y; d <= r; d += 8)
+        if (t < len) {
+            long long s = 0;
+            for (int e = 0; e <= d; ++e) s += sh[e][threadIdx.x];
+            o[(size_t)d * len + t] = s;
+        }
 }
 
 // planes[dz][ky][kx] = sum_dy c(ky, dy) C(kx, w(dy, dz)) for ky <= ny / 2
-__global__ void smv_planes_k(Pair *planes, SmvRows R, const double *__restrict__ cx, const double *__restrict__ cy, size_t nxh,
-                             size_t ny)
+__global__ void smv_planes_k(long long *planes, SmvRows R, const long long *__restrict__ cx, const long long *__restrict__ cy,
+                             size_t nxh, size_t ny)
 {
     const size_t kx = (size_t)blockIdx.x * blockDim.x + threadIdx.x, ky = blockIdx.y, dz = blockIdx.z;
     if (kx >= nxh) return;
-    Pair s{0.0, 0.0};
-    for (int dy = 0; dy < R.ny[dz]; ++dy) s.add(cy[(size_t)dy * ny + ky], cx[(size_t)R.w[dz * SMV_MAX_R + dy] * nxh + kx]);
+    long long s = 0;
+    for (int dy = 0; dy < R.ny[dz]; ++dy) s += __mul64hi(cy[(size_t)dy * ny + ky], cx[(size_t)R.w[dz * SMV_MAX_R + dy] * nxh + kx]);
     planes[(dz * (ny / 2 + 1) + ky) * nxh + kx] = s;
 }
 
-// H and its FP32 copy at (kx, +-ky, +-kz) for ky <= ny / 2, kz <= nz / 2
+// H and its FP32 copy at (kx, +-ky, +-kz) for ky <= ny / 2, kz <= nz / 2; unit: 1 / count over the sums' scale
 template <typename T>
-__global__ void smv_sum_k(T *H, float *H32, const Pair *__restrict__ planes, const double *__restrict__ cz, int rz,
-                          double inv_count, size_t nxh, size_t ny, size_t nz)
+__global__ void smv_sum_k(T *H, float *H32, const long long *__restrict__ planes, const long long *__restrict__ cz, int rz,
+                          double unit, size_t nxh, size_t ny, size_t nz)
 {
     const size_t kx = (size_t)blockIdx.x * blockDim.x + threadIdx.x, ky = blockIdx.y, kz = blockIdx.z;
     if (kx >= nxh) return;
-    Pair s{0.0, 0.0};
-    for (int dz = 0; dz <= rz; ++dz) {
-        const double c = __ldg(cz + (size_t)dz * nz + kz);
-        const Pair p = planes[((size_t)dz * (ny / 2 + 1) + ky) * nxh + kx];
-        s.add(c, p.hi);
-        s.lo = fma(c, p.lo, s.lo);
-    }
-    const T v = (T)((s.hi + s.lo) * inv_count);
+    long long s = 0;
+    for (int dz = 0; dz <= rz; ++dz)
+        s += __mul64hi(__ldg(cz + (size_t)dz * nz + kz), planes[((size_t)dz * (ny / 2 + 1) + ky) * nxh + kx]);
+    const T v = (T)((double)s * unit);
     const size_t yy[2] = {ky, ky ? ny - ky : 0}, zz[2] = {kz, kz ? nz - kz : 0};
     for (int b = 0; b < (zz[1] == zz[0] ? 1 : 2); ++b)
         for (int a = 0; a < (yy[1] == yy[0] ? 1 : 2); ++a) {
@@ -631,21 +650,23 @@ qsm_status smv_direct(qsm_ctx *ctx, Work<T> &w, const Grid &g, const double *h, 
         rows.rz = k;
     }
     // scratch: the row table and the cosines in G, the planes in e
-    const size_t tab = 4096 + ((size_t)(rx + 1) * nxh + (size_t)(ry + 1) * n[1] + (size_t)(rows.rz + 1) * n[2]) * sizeof(double);
-    const size_t pl = (size_t)(rows.rz + 1) * (n[1] / 2 + 1) * nxh * sizeof(Pair);
+    const size_t tab = 4096 + ((size_t)(rx + 1) * nxh + (size_t)(ry + 1) * n[1] + (size_t)(rows.rz + 1) * n[2]) * sizeof(long long);
+    const size_t pl = (size_t)(rows.rz + 1) * (n[1] / 2 + 1) * nxh * sizeof(long long);
     if (tab > g.nh * sizeof(typename Cx<T>::type) || pl > g.p.n() * sizeof(T) || n[1] / 2 + 1 > 65535 || n[2] / 2 + 1 > 65535)
         return QSM_OK;
     char *base = (char *)w.G;
     QSM_CUDA(cudaMemcpyAsync(base, hw, sizeof hw, cudaMemcpyHostToDevice, ctx->stream));  // (pageable: copied before it returns)
     rows.w = (const signed char *)base;
-    double *cx = (double *)(base + 4096), *cy = cx + (size_t)(rx + 1) * nxh, *cz = cy + (size_t)(ry + 1) * n[1];
+    long long *cx = (long long *)(base + 4096), *cy = cx + (size_t)(rx + 1) * nxh, *cz = cy + (size_t)(ry + 1) * n[1];
     const size_t most = std::max(nxh, std::max(n[1], n[2]));
-    smv_tables_k<<<(unsigned)((most + 127) / 128), 128, 0, ctx->stream>>>(cx, cy, cz, n[0], nxh, n[1], n[2], rx, ry, rows.rz);
+    const SmvScale S = smv_scale(rx, ry, rows.rz);
+    smv_tables_k<<<dim3((unsigned)((most + 31) / 32), 3), dim3(32, 8), 0, ctx->stream>>>(cx, cy, cz, n[0], nxh, n[1], n[2], rx, ry,
+                                                                                       rows.rz, S);
     const unsigned gx = (unsigned)((nxh + 127) / 128);
-    smv_planes_k<<<dim3(gx, (unsigned)(n[1] / 2 + 1), (unsigned)(rows.rz + 1)), 128, 0, ctx->stream>>>((Pair *)w.e, rows, cx, cy,
-                                                                                                    nxh, n[1]);
+    smv_planes_k<<<dim3(gx, (unsigned)(n[1] / 2 + 1), (unsigned)(rows.rz + 1)), 128, 0, ctx->stream>>>((long long *)w.e, rows, cx,
+                                                                                                    cy, nxh, n[1]);
     smv_sum_k<T><<<dim3(gx, (unsigned)(n[1] / 2 + 1), (unsigned)(n[2] / 2 + 1)), 128, 0, ctx->stream>>>(
-        w.H, w.H32, (const Pair *)w.e, cz, rows.rz, 1.0 / (double)cnt, nxh, n[1], n[2]);
+        w.H, w.H32, (const long long *)w.e, cz, rows.rz, std::ldexp(1.0 / (double)cnt, -S.v), nxh, n[1], n[2]);
     *done = true;
     return launched(ctx);
 }

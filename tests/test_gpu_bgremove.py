@@ -198,3 +198,17 @@ def test_kept_plans(gpu_ctx, qsm, bg):
                         assert _rel(fl, rfl) <= 1e-9
                 else:
                     assert np.array_equal(fl, first[shape, dt])
+
+
+@pytest.mark.parametrize("shape,vsz,r", [((40, 36, 32), (1.0, 1.0, 1.0), 1.0), ((96, 90, 88), (1.0, 1.0, 1.0), 22.0),
+                                         ((44, 41, 75), (1.0, 1.1, 0.4), 9.0), ((43, 75, 40), (1.5, 0.5, 1.0), 6.3)])
+def test_sphere_spectrum_scales(gpu_ctx, qsm, bg, shape, vsz, r):
+    """The sphere's spectrum in fixed point: one and many offsets an axis, so the
+    smallest and large bounds of its sums, voxels of unequal sides.  FP64 within the
+    filters' bound, eroded masks identical."""
+    f, m = _case(shape, 7)
+    fl, mo = qsm.sharp(f, m, vsz, r, 0.05)
+    rfl, rmo = bg.sharp(f, m, vsz, r, 0.05)
+    assert rmo.any()
+    assert np.array_equal(mo, rmo)
+    assert _rel(fl, rfl) <= 1e-9
