@@ -278,7 +278,7 @@ __global__ void mul_f32_k(cufftComplex *out, const cufftComplex *__restrict__ M,
 __global__ void thresh_k(uint8_t *m, const float *__restrict__ c, float invn, size_t n)
 {
     for (size_t l = (size_t)blockIdx.x * blockDim.x + threadIdx.x; l < n; l += (size_t)gridDim.x * blockDim.x)
-        m[l] = (double)(c[l] * invn) > 0.999 ? 1 : 0;
+        m[l] = c[l] * invn >= 0.999f ? 1 : 0;  // (0.999f is the first single above 0.999)
 }
 
 // F *= (1 - H)  (sharp.m:62-66: h = 1 - h; h .* fft3(f)), or F *= H when one_minus is false
@@ -342,13 +342,26 @@ __global__ void mask_scale_k(T *g, const uint8_t *__restrict__ m, T invn, size_t
         g[l] = (T)(m[l] ? 1 : 0) * (g[l] * invn);
 }
 
-// acc += (mk - mprev) .* (ifft value)  (vsharp.m:124, :143)
+// acc += (mk - mprev) .* (ifft value)  (vsharp.m:124, :143).  Where the masks agree and
+// the value is finite, a zero is added, which changes nothing (acc is never -0): most
+// warps are all such and take no FP64 instruction (out of line: predicated ones would
+// keep their slots; 5.6 M points 46.6 us with them, 16.8 without).
+template <typename T>
+__device__ __noinline__ T vsharp_add(T acc, T g, int diff, T invn)
+{
+    return acc + (T)diff * (g * invn);
+}
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_int(x) & 0x7f800000) == 0x7f800000; }
 template <typename T>
 __global__ void vsharp_acc_k(T *acc, const T *__restrict__ g, const uint8_t *__restrict__ mk,
                              const uint8_t *__restrict__ mprev, T invn, size_t n)
 {
-    for (size_t l = (size_t)blockIdx.x * blockDim.x + threadIdx.x; l < n; l += (size_t)gridDim.x * blockDim.x)
-        acc[l] = acc[l] + ((T)(mk[l] ? 1 : 0) - (T)(mprev[l] ? 1 : 0)) * (g[l] * invn);
+    for (size_t l = (size_t)blockIdx.x * blockDim.x + threadIdx.x; l < n; l += (size_t)gridDim.x * blockDim.x) {
+        const T v = g[l];
+        const int diff = (mk[l] ? 1 : 0) - (mprev[l] ? 1 : 0);
+        if (diff != 0 || not_finite(v)) acc[l] = vsharp_add(acc[l], v, diff, invn);
+    }
 }
 
 template <int NS>

@@ -212,3 +212,17 @@ def test_sphere_spectrum_scales(gpu_ctx, qsm, bg, shape, vsz, r):
     assert rmo.any()
     assert np.array_equal(mo, rmo)
     assert _rel(fl, rfl) <= 1e-9
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_vsharp_not_finite(gpu_ctx, qsm, bg, bad):
+    """A NaN or infinite voxel spreads as in vsharp.m's (m_k - m_(k-1)) .* (...): a zero
+    weight times it is NaN.  The oracle's places, and its masks."""
+    f, m = _case((36, 34, 30), 9)
+    f[tuple(n // 2 for n in f.shape)] = bad
+    with np.errstate(invalid="ignore"):
+        rfl, rmo = bg.vsharp(f, m, [1, 1, 1], [5.0, 3.0], 0.05)
+    fl, mo = qsm.vsharp(f, m, [1, 1, 1], [5.0, 3.0], 0.05)
+    assert np.isnan(rfl).any()
+    assert np.array_equal(mo, rmo)
+    assert np.array_equal(np.isnan(fl), np.isnan(rfl))
