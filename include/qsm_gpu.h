@@ -60,13 +60,17 @@ typedef struct qsm_ctx qsm_ctx;
 
 /* ---------------- context ---------------- */
 
-/* Test hook (no counterpart in the reference).  QSM_DEBUG_GRID_BARRIER_TIMEOUT
+/* Test hooks (no counterpart in the reference).  QSM_DEBUG_GRID_BARRIER_TIMEOUT
  * makes every grid barrier of the whole-GPU multigrid kernels (the coarsest
  * solve and list sweeps on cooperative launches) wait for one arrival more
  * than the grid makes, with a short poll limit, so that their bounded wait
  * runs out: the solve then returns QSM_ERR_TIMEOUT and the context stays
- * usable.  flags = 0 restores normal operation. */
+ * usable.  QSM_DEBUG_WAIT_TIMEOUT does the same for the coarsest solver that
+ * passes values between the CTAs of a cluster: its waits need more bytes than
+ * are sent.  flags = 0 restores normal operation; other bits are refused
+ * (QSM_ERR_ARG). */
 #define QSM_DEBUG_GRID_BARRIER_TIMEOUT 1u
+#define QSM_DEBUG_WAIT_TIMEOUT 4u
 qsm_status qsm_ctx_set_debug(qsm_ctx *ctx, uint32_t flags);
 
 /* Creates a context on `device` with its own non-blocking stream and a

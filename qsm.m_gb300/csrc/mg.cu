@@ -1802,13 +1802,20 @@ static size_t plan_coarse_grid(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c
     return al256(C.n * sizeof(unsigned)) + al256((size_t)(c0 + c1) * sizeof(FlowPkt<T>));
 }
 
-// The slab solver's kernel for a plan's voxels per thread.
+// The slab solver's kernel for a plan's voxels per thread: in FP64 with the multiplies on
+// either pipe (on several CTAs always), in FP32 on one CTA or several.
 template <typename T>
-static const void *slab_kernel(int per, bool soft)
+static const void *slab_kernel(int per, bool soft, bool multi)
 {
-    if (sizeof(T) == 8 && soft)
-        return per == 1 ? (const void *)coarse_slab_k<T, 1, GsK<T>> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsK<T>>;
-    return per == 1 ? (const void *)coarse_slab_k<T, 1, GsC<T>> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsC<T>>;
+    if constexpr (sizeof(T) == 8) {
+        if (soft)
+            return per == 1 ? (const void *)coarse_slab_k<T, 1, GsK<T>, true> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsK<T>, true>;
+        return per == 1 ? (const void *)coarse_slab_k<T, 1, GsC<T>, true> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsC<T>, true>;
+    } else {
+        if (multi)
+            return per == 1 ? (const void *)coarse_slab_k<T, 1, GsC<T>, true> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsC<T>, true>;
+        return per == 1 ? (const void *)coarse_slab_k<T, 1, GsC<T>, false> : (const void *)coarse_slab_k<T, SL_MAX_PER, GsC<T>, false>;
+    }
 }
 
 // The slab solver's dynamic shared-memory limit (as cluster_smem_limit).
@@ -1827,7 +1834,7 @@ static size_t slab_smem_limit(qsm_ctx *ctx)
     size_t l = (size_t)-1;
     for (int v = 0; v < 4; ++v) {
         cudaFuncAttributes fa;
-        const void *k = slab_kernel<T>(v & 1 ? SL_MAX_PER : 1, v & 2);
+        const void *k = slab_kernel<T>(v & 1 ? SL_MAX_PER : 1, v & 2, v & 2);
         if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || (size_t)maxsm <= fa.sharedSizeBytes ||
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)((size_t)maxsm - fa.sharedSizeBytes)) != cudaSuccess ||
@@ -1889,6 +1896,9 @@ static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, cons
     const int ctas = slab_ctas<T>(c0, c1);
     const size_t lim = slab_smem_limit<T>(ctx);
     if (ctas <= 0 || lim == 0) return 0;
+    const bool short_wait = (ctx->debug & QSM_DEBUG_WAIT_TIMEOUT) != 0;
+    t.tries = short_wait ? 64u : SL_TRIES;
+    t.extra = short_wait ? 8u : 0u;
     t.cap = 1;
     for (int c = 0, st = SL_MAX_CTAS / ctas; c < SL_MAX_CTAS; c += st)
         for (int q = 0; q < 2; ++q) t.cap = std::max(t.cap, cut[2 * (c + st) + q] - cut[2 * c + q]);
@@ -1903,7 +1913,7 @@ static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, cons
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = slab_config<T>(t, at);
     int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, slab_kernel<T>(t.per, t.soft), &cfg) != cudaSuccess || ncl < 1) {
+    if (cudaOccupancyMaxActiveClusters(&ncl, slab_kernel<T>(t.per, t.soft, t.ctas > 1), &cfg) != cudaSuccess || ncl < 1) {
         cudaGetLastError();
         t.ctas = 0;
         return 0;
@@ -2322,7 +2332,7 @@ static qsm_status coarse_solve(qsm_ctx *ctx, Hier<T> &H, int l, double *scal_dev
         int *err = H.gb.err, *outer = H.counters;
         void *gc = sizeof(T) == 8 && H.sl.soft ? (void *)&gk : (void *)&gh;
         void *args[] = {&vv, &ff, &rr, &la, &lb, &H.sl, &dd, gc, &lc, &tl, &err, &outer};
-        QSM_CUDA(cudaLaunchKernelExC(&cfg, slab_kernel<T>(H.sl.per, H.sl.soft), args));
+        QSM_CUDA(cudaLaunchKernelExC(&cfg, slab_kernel<T>(H.sl.per, H.sl.soft, H.sl.ctas > 1), args));
         return QSM_OK;
     }
     if (H.cg_ctas > 0) {

@@ -24,6 +24,11 @@
 // first forward pass are of one colour, the former is left out, since the
 // latter recomputes all it wrote from the same values of the other colour.
 //
+// A thread whose wait has run out neither waits nor sends any more, and where it is
+// thread 0 its CTA arms no barrier.  The CTAs that read its values run out in turn.
+// The passes left of the outer iteration run down, then the CTAs leave together after
+// its cluster barrier, with the error word set.
+//
 // Results are those of every other coarsest solver bit for bit: a pass reads
 // the other colour only, so its order is free, and the norm keeps the lane
 // order.  What bounds a pass is latency: a barrier of the CTA's threads (205
@@ -38,7 +43,9 @@ constexpr int SL_MAX_THREADS = 1024;
 constexpr int SL_MAX_PER = 2;                     // voxels of each colour per thread
 constexpr unsigned SL_SOFT_MIN = 256;  // FP64 voxels per colour and CTA from which multiplies leave the FP64 pipe
 constexpr unsigned SL_NONE = 0xFFFFFFFFu;         // pos of a voxel no pass updates
-constexpr long long SL_SPIN_LIMIT = 1ll << 20;
+constexpr unsigned SL_TRY_NS = 2000;              // most one try of a wait is suspended
+constexpr unsigned SL_TRIES = 1u << 20;           // tries before a wait gives up (seconds)
+constexpr unsigned SL_SETTLE_NS = 200000;         // a stopped solver's time for the stores in flight
 
 // meta word of a voxel: export list start (16 bits) and count (3), quirk flags,
 // whether it reads a received value, neighbours read from global memory (6)
@@ -55,6 +62,7 @@ struct SlabTab {
     unsigned cap;  // most voxels of one colour in a chunk
     unsigned win;  // most voxels of one colour within one plane of indices
     size_t smem;
+    unsigned tries, extra;  // a wait's tries; bytes it needs beyond those sent (0; 8 under QSM_DEBUG_WAIT_TIMEOUT)
 };
 
 // Shared-memory layout of one CTA (host and device agree on it).
@@ -125,20 +133,41 @@ __device__ __forceinline__ void sl_arm(uint32_t mb, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes) : "memory");
 }
-// waits for the phase of this parity; false once the wait has run out
-__device__ __forceinline__ bool sl_wait(uint32_t mb, uint32_t parity)
+// waits for the phase of this parity; false once the tries, each of bounded time, have run out
+__device__ __forceinline__ bool sl_wait(uint32_t mb, uint32_t parity, unsigned tries)
 {
-    for (long long tries = 0; tries < SL_SPIN_LIMIT; ++tries) {
+    for (unsigned k = 0; k < tries; ++k) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok)
-                     : "r"(mb), "r"(parity)
+                     : "r"(mb), "r"(parity), "r"(SL_TRY_NS)
                      : "memory");
         if (ok) return true;
     }
     return false;
+}
+
+// Sets the stop word of every CTA.
+__device__ __noinline__ void sl_stop(unsigned *stop)
+{
+    const uint32_t cn = cl_size();
+    for (uint32_t r = 0; r < cn; ++r) cl_or(cl_map(stop, r), 1u);
+}
+
+// Time for the stores of a stopped solver to land, whose barriers no longer tell: none
+// is sent any more, and one takes under a microsecond.  (The reads of the clock are
+// bounded too.)
+__device__ __noinline__ void sl_settle()
+{
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (int k = 0; k < (1 << 16); ++k) {
+        __nanosleep(1000);
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 >= SL_SETTLE_NS) break;
+    }
 }
 
 // lane-order sum of src[e]^2 over e < n <= RED_LANES (src in global memory,
@@ -220,16 +249,16 @@ __device__ __forceinline__ void slab_globals(T (&x)[6], uint32_t g, const T *gv,
 // in FP32 their meta word, SL_ON alone, takes a short way.  FP64 has one way
 // only: a warp with voxels of both kinds would issue the update twice, and an
 // FP64 instruction costs its ~80 cycles whatever lanes it has.
-template <typename T, int PER, typename GC>
+template <typename T, int PER, typename GC, bool MULTI>
 __device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const SlabCol &C, uint32_t skip, const GC &c,
                                           const T *gv, int nx, int nxny, uint32_t wait_mb, uint32_t wait_par, bool wait,
-                                          int &dead)
+                                          unsigned tries, int &dead, int &arm)
 {
     const uint32_t step = blockDim.x * (uint32_t)sizeof(T);
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
         const uint32_t meta = S.meta[u];
-        if (meta == 0) continue;
+        if (sizeof(T) == 4 && meta == 0) continue;
         if (sizeof(T) == 4 && (meta & (~(SL_I1 | SL_INX2) | skip)) == SL_ON) {
             T x[6];
 #pragma unroll
@@ -237,7 +266,14 @@ __device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const Slab
             sl_st(C.own + u * step, c.hh * (S.f[u] + (c.hx * (x[0] + x[1]) + c.hy * (x[2] + x[3]) + c.hz * (x[4] + x[5]))));
             continue;
         }
-        if (wait && (meta & SL_HALO) && !dead && !sl_wait(wait_mb, wait_par)) dead = 1;
+        if (MULTI && wait && (meta & SL_HALO) && !dead && !sl_wait(wait_mb, wait_par, tries)) {
+            dead = 1;
+            arm = 0;
+        }
+        if (sizeof(T) == 8) {
+            __syncwarp();  // (else compiled as two ways after all: 64^3 with two levels 34.4 instead of 28.5 ms)
+            if (meta == 0) continue;
+        }
         T val;
         if (meta & skip) {
             val = sl_ld(C.own + u * step, T());
@@ -250,7 +286,7 @@ __device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const Slab
             val = c.hh * (S.f[u] + (c.hx * (x[0] + x[1]) + c.hy * (x[2] + x[3]) + c.hz * (x[4] + x[5])));
             sl_st(C.own + u * step, val);
         }
-        const unsigned cnt = (meta >> 16) & 7u, s0 = meta & 0xffffu;
+        const unsigned cnt = !MULTI || dead ? 0u : (meta >> 16) & 7u, s0 = meta & 0xffffu;
         for (unsigned k = 0; k < cnt; ++k) {
             const uint32_t t = C.exp[s0 + k];
             sl_send(sl_mapa(C.va, t >> 16) + (t & 0xffffu) * (uint32_t)sizeof(T), val, sl_mapa(C.mb, t >> 16));
@@ -259,7 +295,9 @@ __device__ __forceinline__ void slab_pass(const SlabShare<T, PER> &S, const Slab
     __syncthreads();
 }
 
-template <typename T, int PER, typename GC>
+// MULTI: more than one CTA (one alone without the code of waits and sends: FP32 64^3 with
+// four levels 2.05 instead of 2.17 ms)
+template <typename T, int PER, typename GC, bool MULTI>
 __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *__restrict__ gf, T *gr,
                                                                 const uint32_t *__restrict__ l0,
                                                                 const uint32_t *__restrict__ l1, SlabTab tab, Dims d,
@@ -268,10 +306,10 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ __align__(8) unsigned long long mbar[2];
-    __shared__ unsigned bnd[2 * (SL_MAX_CTAS + 1)], nexp[2], nrecv[2], cflag;
+    __shared__ unsigned bnd[2 * (SL_MAX_CTAS + 1)], nexp[2], nrecv[2], cflag, stop;
     const SlabLayout lay(tab.cap, tab.win, tab.ctas, sizeof(T));
     const unsigned win = tab.win, len = lay.len;
-    const uint32_t c = cl_rank(), cn = cl_size();
+    const uint32_t c = MULTI ? cl_rank() : 0u, cn = MULTI ? cl_size() : 1u;
     const int nx = (int)d.nx, nxny = (int)d.nxny();
     const unsigned n = (unsigned)d.n();
     const int tid = (int)threadIdx.x;
@@ -288,6 +326,7 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     }
     if (tid == 0) {
         cflag = 0;
+        stop = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int t = tid; t < RED_NBLK; t += blockDim.x) blk[t] = (T)0;
@@ -295,8 +334,10 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     if (cn > 1)
         for (unsigned t = tid; t < 2 * len; t += blockDim.x) need[t] = 0;
     chain_wait();
+    const int failed = *(const volatile int *)err;
     for (int t = tid; t < 2 * ((int)cn + 1); t += blockDim.x) bnd[t] = tab.cut[2 * (t / 2 * (SL_MAX_CTAS / (int)cn)) + t % 2];
     __syncthreads();
+    if (failed) return;  // an earlier wait ran out (the whole cluster reads the same)
     const unsigned start[2] = {bnd[2 * c], bnd[2 * c + 1]};
     const unsigned cnt[2] = {bnd[2 * c + 2] - start[0], bnd[2 * c + 3] - start[1]};
     list[0] += start[0];
@@ -385,7 +426,14 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     }
     // every chunk has loaded the values around it (and its barriers are set) before any is sent
     cl_sync();
-    const uint32_t bytes[2] = {nrecv[0] * (uint32_t)sizeof(T), nrecv[1] * (uint32_t)sizeof(T)};
+    uint32_t bytes[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        bytes[q] = nrecv[q] ? nrecv[q] * (uint32_t)sizeof(T) + tab.extra : 0u;
+        // thread 0 waits for every phase that bytes complete (SL_PASS says why); it has a
+        // voxel then, as one of the other colour reads those
+        if (tid == 0 && nrecv[q]) S[q ^ 1].meta[0] |= SL_HALO;
+    }
     const uint32_t mb[2] = {sl_addr(&mbar[0]), sl_addr(&mbar[1])};
     const SlabCol col[2] = {{va[0] + (win + tid) * (uint32_t)sizeof(T), va[0], mb[0], exp[0], list[0]},
                             {va[1] + (win + tid) * (uint32_t)sizeof(T), va[1], mb[1], exp[1], list[1]}};
@@ -401,16 +449,19 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
     const bool idle = cflag != 3u;
     const bool r1first = ((nx + 1) & 1) != 0;  // reverse sweeps begin with colour 1
     unsigned done[2] = {0, 0};                 // passes of each colour so far
-    int dead = 0;
-    // one pass of colour Q: reads the other colour's values of its last pass
+    int dead = 0, arm = cn > 1 && tid == 0;
+    // one pass of colour Q: reads the other colour's values of its last pass.  Thread 0
+    // arms the barrier of Q's values.  It has waited itself for that barrier's last phase,
+    // in the pass before (SL_HALO is set for it): a phase still open must not be armed.
 #define SL_PASS(Q, SKIP)                                                                                            \
     do {                                                                                                            \
-        if (cn > 1 && tid == 0) sl_arm(mb[Q], bytes[Q]);                                                            \
-        slab_pass<T, PER, GC>(S[Q], col[Q], SKIP, gc, gv, nx, nxny, mb[1 - (Q)], (done[1 - (Q)] - 1) & 1u,              \
-                          done[1 - (Q)] > 0, dead);                                                                 \
+        if (MULTI && arm) sl_arm(mb[Q], bytes[Q]);                                                                  \
+        slab_pass<T, PER, GC, MULTI>(S[Q], col[Q], SKIP, gc, gv, nx, nxny, mb[1 - (Q)], (done[1 - (Q)] - 1) & 1u,              \
+                          done[1 - (Q)] > 0, tab.tries, dead, arm);                                                 \
         ++done[Q];                                                                                                  \
     } while (0)
     int outer = 0;
+    bool stopped = false;
     for (int it = 0; it < 1024; ++it) {
         outer = it + 1;
         if (r1first) {
@@ -430,8 +481,9 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
             SL_PASS(1, SL_I1);
         }
         if (cn > 1 && !dead) {
-            if (!sl_wait(mb[0], (done[0] - 1) & 1u) || !sl_wait(mb[1], (done[1] - 1) & 1u)) dead = 1;
+            if (!sl_wait(mb[0], (done[0] - 1) & 1u, tab.tries) || !sl_wait(mb[1], (done[1] - 1) & 1u, tab.tries)) dead = 1;
         }
+        if (dead) sl_stop(&stop);
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -449,6 +501,11 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
             }
         }
         cl_sync();
+        if (cn > 1 && *(volatile unsigned *)&stop) {  // (the same in every CTA: set before its setter arrived)
+            stopped = true;
+            sl_settle();
+            break;
+        }
         const T rr = sl_lane_sum(gr, n, blk, bc, c, cn);
         const double rn = sizeof(T) == 4 ? (double)sqrtf((float)rr) : sqrt((double)rr);
         if (rn < reltol) break;
@@ -466,7 +523,7 @@ __global__ void __launch_bounds__(SL_MAX_THREADS) coarse_slab_k(T *gv, const T *
                 const unsigned e = (unsigned)tid + u * blockDim.x;
                 gv[list[q][e] & BL_IDX] = v[q][win + e];
             }
-    if (dead) atomicExch(err, 1);
+    if (stopped && tid == 0) atomicExch(err, 1);
     if (c == 0 && tid == 0 && outer_out) *outer_out += outer;
     cl_sync();  // no CTA leaves while a peer may still address its shared memory
 }

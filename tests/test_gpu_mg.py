@@ -270,6 +270,40 @@ def test_grid_barrier_wait_runs_out(gpu_ctx, qsm, port):
     assert bits_equal(a, b), first_diff(a, b)
 
 
+@pytest.mark.parametrize("dt,shape,nl", [("float64", (30, 28, 26), 1), ("float32", (44, 40, 38), 1)])
+def test_coarsest_value_waits_run_out(gpu_ctx, qsm, port, dt, shape, nl):
+    """The waits of the coarsest solver whose CTAs pass values to each other in a
+    cluster.  Under the context's test hook each needs more bytes than are ever sent
+    and gives up soon: the solve must return QSM_ERR_TIMEOUT within seconds, every
+    CTA leaving together, and the same context must then solve bit for bit against
+    the oracle."""
+    import time
+
+    import qsm_gb300._lib as _lib
+    import qsm_gb300.synthetic as S
+
+    f, m, _ = S.poisson_case(shape, 31, semi=(0.3 * min(shape), 0.45 * min(shape)))
+    f = np.asfortranarray(f.astype(dt))
+    v0 = np.zeros(shape, dtype=dt, order="F")
+    args = ([1, 1, 1], -1.0, 1, 1, 2, 2, 2, nl)
+    L = _lib.lib()
+    assert L.qsm_ctx_set_debug(gpu_ctx.handle, 4) == 0
+    try:
+        t0 = time.perf_counter()
+        with pytest.raises(_lib.QsmError) as ei:
+            qsm.mg_mex(v0, f, m, *args, ctx=gpu_ctx)
+        assert ei.value.status == 9  # QSM_ERR_TIMEOUT
+        with pytest.raises(_lib.QsmError) as ei:
+            qsm.mgpcg_mex(v0, f, m, [1, 1, 1], 1e-8, 5, -1.0, 2, 1, 2, 2, 2, nl, ctx=gpu_ctx)
+        assert ei.value.status == 9
+        assert time.perf_counter() - t0 < 20
+    finally:
+        assert L.qsm_ctx_set_debug(gpu_ctx.handle, 0) == 0
+    a = qsm.mg_mex(v0, f, m, *args, ctx=gpu_ctx)
+    b = port.mg_mex(v0, f, m, *args)
+    assert bits_equal(a, b), first_diff(a, b)
+
+
 @pytest.mark.parametrize("dt", ("float64", "float32"))
 def test_mgpcg_256_lbv_options_bitexact(gpu_ctx, qsm, port, dt):
     """The benchmark's Poisson problem at full size (256^3, LBV options, 5
