@@ -65,10 +65,10 @@ typedef struct qsm_ctx qsm_ctx;
  * solve and list sweeps on cooperative launches) wait for one arrival more
  * than the grid makes, with a short poll limit, so that their bounded wait
  * runs out: the solve then returns QSM_ERR_TIMEOUT and the context stays
- * usable.  QSM_DEBUG_WAIT_TIMEOUT does the same for the coarsest solver that
- * passes values between the CTAs of a cluster: its waits need more bytes than
- * are sent.  flags = 0 restores normal operation; other bits are refused
- * (QSM_ERR_ARG). */
+ * usable.  QSM_DEBUG_WAIT_TIMEOUT does the same for the coarsest solvers that
+ * pass values between CTAs: the waits of a cluster need more bytes than are
+ * sent, the polls of packets a pass that is never run.  flags = 0 restores
+ * normal operation; other bits are refused (QSM_ERR_ARG). */
 #define QSM_DEBUG_GRID_BARRIER_TIMEOUT 1u
 #define QSM_DEBUG_WAIT_TIMEOUT 4u
 qsm_status qsm_ctx_set_debug(qsm_ctx *ctx, uint32_t flags);

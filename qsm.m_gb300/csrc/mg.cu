@@ -760,10 +760,12 @@ constexpr long long CG_SPIN_LIMIT = 1ll << 22;  // polls of the generation word 
 constexpr unsigned CG_MIN_PASS = 6000;          // per-colour G count from which the grid beats a cluster
 
 struct GridBar {
-    unsigned *count;  // arrivals since the launch (zeroed by the host before it)
+    unsigned *count;  // arrivals since the host zeroed it, before the launch or the first of several that count on
     int *err;
     unsigned extra;   // arrivals required beyond the grid's (0; 1 under QSM_DEBUG_GRID_BARRIER_TIMEOUT)
     long long limit;  // polls before a wait gives up
+    int polls;        // of a packet (mg_flow.cuh) before a wait gives up
+    unsigned ahead;   // passes by which a packet must be later than needed (0; never reached under QSM_DEBUG_WAIT_TIMEOUT)
 };
 
 // Barrier number k (1, 2, ...) of the grid: each CTA adds one arrival with
@@ -1734,6 +1736,9 @@ static qsm_status hier_init(qsm_ctx *ctx, Hier<T> &H, int nl, const Dims &dp, co
     const bool short_bar = (ctx->debug & QSM_DEBUG_GRID_BARRIER_TIMEOUT) != 0;
     H.gb.extra = short_bar ? 1u : 0u;
     H.gb.limit = short_bar ? (1ll << 12) : CG_SPIN_LIMIT;
+    const bool short_wait = (ctx->debug & QSM_DEBUG_WAIT_TIMEOUT) != 0;
+    H.gb.polls = short_wait ? 1 << 10 : FL_SPIN_LIMIT;
+    H.gb.ahead = short_wait ? 1u << 28 : 0u;
     const size_t nc = H.L[nl - 1].n;
     H.coarse_smem = cs_smem(nc, sizeof(T)) + 64;
     int maxsm = 0;

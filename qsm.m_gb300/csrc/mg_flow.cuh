@@ -31,7 +31,7 @@
 // grid.  Measured: see plan_coarse_grid.
 
 constexpr int FL_THREADS = 512;  // most threads of a CTA, one voxel of each colour per thread
-constexpr int FL_SPIN_LIMIT = 1 << 20;
+constexpr int FL_SPIN_LIMIT = 1 << 20;  // polls of a packet before a wait gives up (seconds)
 
 // What the two passes of step s = 0 .. 255 of an outer iteration leave out: its
 // 128 reverse and 128 forward sweeps as strictly alternating passes.  With
@@ -123,7 +123,7 @@ __device__ __forceinline__ T flow_local(const FlowVox<T> &V, int k, const T *gv,
 template <typename T>
 __device__ __forceinline__ void flow_pass(const FlowVox<T> &V, uint32_t own, uint32_t skip, const GsC<T> &c, const T *gv,
                                           FlowPkt<T> *po, const FlowPkt<T> *pn, int nx, int nxny, unsigned need,
-                                          unsigned tag, int &dead)
+                                          unsigned tag, int polls, int &dead)
 {
     if (V.meta & FL_ON) {
         T val;
@@ -151,7 +151,7 @@ __device__ __forceinline__ void flow_pass(const FlowVox<T> &V, uint32_t own, uin
                         pend &= ~(1u << k);
                     }
                 if (!pend) break;
-                if (++tries > FL_SPIN_LIMIT) dead = 1;
+                if (++tries > polls) dead = 1;
 #pragma unroll
                 for (int k = 0; k < 6; ++k)
                     if (pend >> k & 1u) fl_get(pn + V.a[k], y[k], tg[k]);
@@ -248,10 +248,10 @@ __global__ void __launch_bounds__(FL_THREADS) coarse_flow_k(T *v, const T *__res
         outer = it + 1;
         for (int s = 0; s < 256; ++s) {
             const SweepSkip k = sweep_skip(r1first, s, FL_I1, FL_INX2);
-            flow_pass<T>(V[0], own[0], k.first, gc, v, pk0, pk1, nx, nxny, last1, ++tag, dead);
+            flow_pass<T>(V[0], own[0], k.first, gc, v, pk0, pk1, nx, nxny, last1 + gb.ahead, ++tag, gb.polls, dead);
             last0 = tag;
             if (k.only_first) break;
-            flow_pass<T>(V[1], own[1], k.second, gc, v, pk1, pk0, nx, nxny, last0, ++tag, dead);
+            flow_pass<T>(V[1], own[1], k.second, gc, v, pk1, pk0, nx, nxny, last0 + gb.ahead, ++tag, gb.polls, dead);
             last1 = tag;
         }
 #pragma unroll

@@ -270,19 +270,23 @@ def test_grid_barrier_wait_runs_out(gpu_ctx, qsm, port):
     assert bits_equal(a, b), first_diff(a, b)
 
 
-@pytest.mark.parametrize("dt,shape,nl", [("float64", (30, 28, 26), 1), ("float32", (44, 40, 38), 1)])
-def test_coarsest_value_waits_run_out(gpu_ctx, qsm, port, dt, shape, nl):
-    """The waits of the coarsest solver whose CTAs pass values to each other in a
-    cluster.  Under the context's test hook each needs more bytes than are ever sent
-    and gives up soon: the solve must return QSM_ERR_TIMEOUT within seconds, every
-    CTA leaving together, and the same context must then solve bit for bit against
-    the oracle."""
+@pytest.mark.parametrize("dt,shape,nl,plates", [("float64", (30, 28, 26), 1, False), ("float32", (44, 40, 38), 1, False),
+                                                ("float64", (96, 88, 80), 2, False), ("float32", (66, 64, 64), 1, True)])
+def test_coarsest_value_waits_run_out(gpu_ctx, qsm, port, dt, shape, nl, plates):
+    """The waits of the coarsest solvers whose CTAs pass values to each other: in a
+    cluster (the first two cases) and as packets over the whole GPU.  Under the
+    context's test hook each needs what is never sent and gives up soon: the solve
+    must return QSM_ERR_TIMEOUT within seconds, every CTA leaving together, and the
+    same context must then solve bit for bit against the oracle."""
     import time
 
     import qsm_gb300._lib as _lib
     import qsm_gb300.synthetic as S
 
-    f, m, _ = S.poisson_case(shape, 31, semi=(0.3 * min(shape), 0.45 * min(shape)))
+    f, m, _ = S.poisson_case(shape, 31, semi=(0.36 * min(shape), 0.48 * min(shape)))
+    if plates:
+        m = np.asfortranarray(np.broadcast_to(np.arange(shape[2]) % 4 == 1, shape).astype(np.uint8))
+        f = np.asfortranarray(np.random.default_rng(32).standard_normal(shape) * m)
     f = np.asfortranarray(f.astype(dt))
     v0 = np.zeros(shape, dtype=dt, order="F")
     args = ([1, 1, 1], -1.0, 1, 1, 2, 2, 2, nl)
