@@ -273,15 +273,25 @@ qsm_status qsm_norm2_noalloc(qsm_dtype dtype, size_t n, const void *x, const uin
 
 /* ---------------- Poisson solvers ---------------- */
 
+/* The coarsest-level solver of a multigrid solve (qsm_mg_info.coarse_solver). */
+enum {
+    QSM_COARSE_HOST = 0,     /* the loop driven from the host */
+    QSM_COARSE_ONE_CTA = 1,  /* one CTA per solve, values in shared memory */
+    QSM_COARSE_SLABS = 2,    /* planes over a cluster, a cluster barrier per pass */
+    QSM_COARSE_CHUNKS = 3,   /* voxel lists over one CTA or a cluster, values sent where they are read */
+    QSM_COARSE_PACKETS = 4,  /* voxel lists over the whole GPU (cooperative), values as packets */
+    QSM_COARSE_BARRIERS = 5  /* the same with a grid barrier per pass */
+};
+
 typedef struct {
     int32_t iters;          /* PCG iterations (mgpcg) or cycles run */
+    int32_t coarse_solver;  /* QSM_COARSE_*: which coarsest-level solver ran */
     double resnorm;         /* final ||r||_2 (padded array, as the reference) */
     double seconds;         /* device time */
     double *resnorm_hist;   /* optional, caller-owned, >= maxitcg doubles */
-    int32_t coarse_ctas;    /* coarsest-level solver: 0 host-driven loop, 1 one CTA,
-                               > 1 a thread-block cluster of that many CTAs, < 0
-                               (passes of more than 6000 voxels) -coarse_ctas CTAs, one
-                               per SM: a cooperative launch in FP64, a cluster in FP32 */
+    int32_t coarse_ctas;    /* its CTAs, 0 for the host-driven loop; negative where a
+                               colour has more than 6000 voxels, whichever solver ran
+                               (in FP32 often a cluster), and for the cooperative ones */
     int32_t coarse_outer;   /* outer iterations (256 sweeps each) it ran in total */
 } qsm_mg_info;
 

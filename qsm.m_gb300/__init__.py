@@ -343,6 +343,10 @@ def fp_convert_check(*, ctx=None) -> int:
 # Poisson solvers
 # ---------------------------------------------------------------------------
 
+# qsm_mg_info.coarse_solver (QSM_COARSE_*)
+_COARSE = ("host", "one CTA", "slabs", "chunks", "packets", "barriers")
+
+
 def mgpcg_mex(v, f, mask, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, npost, nboundary, nlevels, verbose=0,
               *, mixed=False, info=None, ctx=None):
     """v = mgpcg_mex(v, f, mask, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, npost, nboundary, nlevels, verbose).
@@ -370,7 +374,8 @@ def mgpcg_mex(v, f, mask, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, npost, 
                        int(verbose), o.ptr, ctypes.byref(mi))
     if info is not None:
         info.update(iters=mi.iters, resnorm=mi.resnorm, seconds=mi.seconds, resnorm_hist=hist[: mi.iters].copy(),
-                    coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer)
+                    coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer,
+                    coarse_solver=_COARSE[mi.coarse_solver])
     return out
 
 
@@ -386,7 +391,8 @@ def mg_mex(v, f, mask, vsz, tol, maxit, mu, npre, npost, nboundary, nlevels, *, 
                    float(tol), int(maxit), int(mu), int(npre), int(npost), int(nboundary), int(nlevels), o.ptr,
                    ctypes.byref(mi))
     if info is not None:
-        info.update(cycles=mi.iters, seconds=mi.seconds, coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer)
+        info.update(cycles=mi.iters, seconds=mi.seconds, coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer,
+                    coarse_solver=_COARSE[mi.coarse_solver])
     return out
 
 
@@ -400,7 +406,8 @@ def fmg_mex(f, mask, vsz, tol, maxit, mu, npre, npost, nboundary, nlevels, *, in
     _ctx(ctx).call("qsm_fmg", fa.dt, fa.dims_c(), fa.ptr, m.ptr, _h(vsz), float(tol), int(maxit), int(mu),
                    int(npre), int(npost), int(nboundary), int(nlevels), o.ptr, ctypes.byref(mi))
     if info is not None:
-        info.update(cycles=mi.iters, seconds=mi.seconds, coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer)
+        info.update(cycles=mi.iters, seconds=mi.seconds, coarse_ctas=mi.coarse_ctas, coarse_outer=mi.coarse_outer,
+                    coarse_solver=_COARSE[mi.coarse_solver])
     return out
 
 
@@ -492,7 +499,8 @@ def lbv(f, mask, vsz, tol=1e-8, maxit=None, mgopts=None, verbose=0, *, mixed=Fal
                    mis)
     if infos is not None:
         infos[:] = [dict(iters=mis[t].iters, resnorm=mis[t].resnorm, seconds=mis[t].seconds,
-                         coarse_ctas=mis[t].coarse_ctas, coarse_outer=mis[t].coarse_outer) for t in range(ne)]
+                         coarse_ctas=mis[t].coarse_ctas, coarse_outer=mis[t].coarse_outer,
+                         coarse_solver=_COARSE[mis[t].coarse_solver]) for t in range(ne)]
     return out
 
 
@@ -673,7 +681,8 @@ def mgpcg_batch(v0s, fs, masks, vsz, tolcg, maxitcg, tolmg, maxitmg, mu, npre, n
     if infos is not None:
         infos[:] = [dict(iters=mis[b].iters, resnorm=mis[b].resnorm, seconds=mis[b].seconds,
                          resnorm_hist=hists[b][: mis[b].iters].copy(), coarse_ctas=mis[b].coarse_ctas,
-                         coarse_outer=mis[b].coarse_outer) for b in range(n)]
+                         coarse_outer=mis[b].coarse_outer, coarse_solver=_COARSE[mis[b].coarse_solver])
+                    for b in range(n)]
     return outs
 
 

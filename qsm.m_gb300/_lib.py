@@ -56,9 +56,9 @@ class TvInfo(ctypes.Structure):
 
 
 class MgInfo(ctypes.Structure):
-    _fields_ = [("iters", ctypes.c_int32), ("resnorm", ctypes.c_double), ("seconds", ctypes.c_double),
-                ("resnorm_hist", ctypes.POINTER(ctypes.c_double)), ("coarse_ctas", ctypes.c_int32),
-                ("coarse_outer", ctypes.c_int32)]
+    _fields_ = [("iters", ctypes.c_int32), ("coarse_solver", ctypes.c_int32), ("resnorm", ctypes.c_double),
+                ("seconds", ctypes.c_double), ("resnorm_hist", ctypes.POINTER(ctypes.c_double)),
+                ("coarse_ctas", ctypes.c_int32), ("coarse_outer", ctypes.c_int32)]
 
 
 class NiftiHdr(ctypes.Structure):

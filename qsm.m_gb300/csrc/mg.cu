@@ -2924,6 +2924,8 @@ static qsm_status coarse_report(qsm_ctx *ctx, const Hier<T> &H, qsm_mg_info *inf
         }
     }
     if (!info) return QSM_OK;
+    info->coarse_solver = H.sl.ctas > 0 ? QSM_COARSE_CHUNKS : H.cg_ctas > 0 ? (H.cg_threads > 0 ? QSM_COARSE_PACKETS : QSM_COARSE_BARRIERS)
+                        : H.cc_ctas > 0 ? QSM_COARSE_SLABS : H.coarse_in_smem ? QSM_COARSE_ONE_CTA : QSM_COARSE_HOST;
     int dev_outer = 0;
     QSM_CUDA(cudaMemcpy(&dev_outer, H.counters, sizeof(int), cudaMemcpyDeviceToHost));
     info->coarse_ctas = H.sl.ctas > 0 ? (H.sl_large ? -H.sl.ctas : H.sl.ctas) : H.cg_ctas > 0 ? -H.cg_ctas : H.cc_ctas > 0 ? H.cc_ctas : (H.coarse_in_smem ? 1 : 0);

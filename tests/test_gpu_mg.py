@@ -514,3 +514,25 @@ def test_cycles_reuse_levels_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl):
         b = port.fmg_mex(f, m, [1, 1, 1], -1.0, 2, mu, 1, 2, 2, nl)
         a = qsm.fmg_mex(f, m, [1, 1, 1], -1.0, 2, mu, 1, 2, 2, nl)
         assert bits_equal(a, b), first_diff(a, b)
+
+
+@pytest.mark.parametrize("dt,shape,nl,solver,ctas", [("float32", (62, 62, 62), 3, "chunks", 1), ("float64", (62, 62, 62), 3, "chunks", 16),
+                                                     ("float32", (96, 88, 80), 2, "chunks", -16), ("float64", (96, 88, 80), 2, "packets", 0)])
+def test_reported_coarsest_solver(gpu_ctx, qsm, dt, shape, nl, solver, ctas):
+    """coarse_solver names the solver that ran; the sign of coarse_ctas does not: an
+    FP32 solve with more than 6000 voxels a colour runs on a cluster (-16), an FP64
+    one over the whole GPU (ctas 0 here: minus the SMs).  Packed solves run on one
+    CTA each."""
+    import qsm_gb300.synthetic as S
+    import torch
+
+    f, m, _ = S.poisson_case(shape, 9, semi=(0.31 * shape[0], 0.42 * shape[0]))
+    f = np.asfortranarray(f.astype(dt))
+    gi = {}
+    qsm.mg_mex(None, f, m, [1, 1, 1], -1.0, 1, 1, 2, 2, 2, nl, info=gi)
+    want = ctas or -torch.cuda.get_device_properties(0).multi_processor_count
+    assert (gi["coarse_solver"], gi["coarse_ctas"]) == (solver, want)
+    if dt == "float64" and nl == 3:
+        infos = []
+        qsm.mgpcg_batch(None, [f, f], [m, m], [1, 1, 1], 1e-8, 2, -1.0, 2, 1, 2, 2, 2, nl, infos=infos)
+        assert [(i["coarse_solver"], i["coarse_ctas"]) for i in infos] == [("one CTA", 1)] * 2
