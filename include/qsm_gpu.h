@@ -67,10 +67,13 @@ typedef struct qsm_ctx qsm_ctx;
  * runs out: the solve then returns QSM_ERR_TIMEOUT and the context stays
  * usable.  QSM_DEBUG_WAIT_TIMEOUT does the same for the coarsest solvers that
  * pass values between CTAs: the waits of a cluster need more bytes than are
- * sent, the polls of packets a pass that is never run.  flags = 0 restores
- * normal operation; other bits are refused (QSM_ERR_ARG). */
+ * sent, the polls of packets a pass that is never run.  QSM_DEBUG_NO_LISTS
+ * makes multigrid solves run without voxel lists, as on grids of 2^30 voxels or
+ * more: full-grid passes, and the coarsest solvers that need no lists.
+ * flags = 0 restores normal operation; other bits are refused (QSM_ERR_ARG). */
 #define QSM_DEBUG_GRID_BARRIER_TIMEOUT 1u
 #define QSM_DEBUG_WAIT_TIMEOUT 4u
+#define QSM_DEBUG_NO_LISTS 8u
 qsm_status qsm_ctx_set_debug(qsm_ctx *ctx, uint32_t flags);
 
 /* Creates a context on `device` with its own non-blocking stream and a

@@ -352,7 +352,7 @@ qsm_status qsm_ctx_create(int device, qsm_ctx **out)
 qsm_status qsm_ctx_set_debug(qsm_ctx *ctx, uint32_t flags)
 {
     if (!ctx) return QSM_ERR_ARG;
-    if (flags & ~(uint32_t)(QSM_DEBUG_GRID_BARRIER_TIMEOUT | QSM_DEBUG_WAIT_TIMEOUT)) return QSM_ERR_ARG;
+    if (flags & ~(uint32_t)(QSM_DEBUG_GRID_BARRIER_TIMEOUT | QSM_DEBUG_WAIT_TIMEOUT | QSM_DEBUG_NO_LISTS)) return QSM_ERR_ARG;
     ctx->debug = flags;
     return QSM_OK;
 }

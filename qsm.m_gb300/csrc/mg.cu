@@ -1933,7 +1933,7 @@ static size_t plan_slab(qsm_ctx *ctx, Hier<T> &H, unsigned c0, unsigned c1, cons
 template <typename T>
 static qsm_status boundary_lists(qsm_ctx *ctx, Hier<T> &H)
 {
-    if (H.L[0].n >= ((size_t)1 << 30)) return QSM_OK;
+    if (H.L[0].n >= ((size_t)1 << 30) || (ctx->debug & QSM_DEBUG_NO_LISTS)) return QSM_OK;
     const int cn = sweeps_cluster_size<T>(ctx);
     unsigned *cnt = (unsigned *)H.counters + 8;  // B: 4i, 4i+1; G: 4i+2, 4i+3 (nl <= 16)
     const int ncnt = 4 * H.nl + 2 * (SL_MAX_CTAS + 1);  // then the coarsest level's cuts

@@ -536,3 +536,55 @@ def test_reported_coarsest_solver(gpu_ctx, qsm, dt, shape, nl, solver, ctas):
         infos = []
         qsm.mgpcg_batch(None, [f, f], [m, m], [1, 1, 1], 1e-8, 2, -1.0, 2, 1, 2, 2, 2, nl, infos=infos)
         assert [(i["coarse_solver"], i["coarse_ctas"]) for i in infos] == [("one CTA", 1)] * 2
+
+
+@pytest.mark.parametrize("dt", ("float64", "float32"))
+@pytest.mark.parametrize("nx", (58, 59))
+def test_coarsest_grid_barriers_vs_oracle(gpu_ctx, qsm, port, dt, nx):
+    """More voxels a colour than the packet solver's CTAs have threads (512 per SM):
+    the solver with a grid barrier per pass, whose norm sums two elements per lane
+    here, for both parities of nx.  Bit-for-bit against the oracle."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ny = 50
+    nz = 2 * (512 * sms * 21 // 20) // (nx * ny) + 1
+    shape = (nx, ny, nz)
+    rng = np.random.default_rng(nx)
+    m = np.ones(shape, np.uint8, order="F")
+    f = np.asfortranarray(rng.standard_normal(shape).astype(dt))
+    v0 = np.zeros(shape, order="F", dtype=dt)
+    h = [1, 0.9, 1.2]
+    gi = {}
+    a = qsm.mg_mex(v0, f, m, h, -1.0, 1, 1, 1, 1, 1, 1, info=gi)
+    assert gi["coarse_solver"] == "barriers"
+    b = port.mg_mex(v0, f, m, h, -1.0, 1, 1, 1, 1, 1, 1)
+    assert bits_equal(a, b), first_diff(a, b)
+
+
+@pytest.mark.parametrize("dt,shape,nl,solver", [("float64", (30, 28, 26), 1, "slabs"), ("float64", (62, 60, 44), 2, "slabs"),
+                                                ("float64", (60, 58, 56), 1, "host"), ("float32", (48, 44, 40), 3, "one CTA"),
+                                                ("float32", (40, 36, 45), 2, "one CTA"), ("float32", (33, 41, 30), 1, "slabs")])
+def test_no_lists_vs_oracle(gpu_ctx, qsm, port, dt, shape, nl, solver):
+    """Without voxel lists (grids of 2^30 voxels or more, here by the test hook): the
+    coarsest solvers that need none, and full-grid passes.  Bit-for-bit against the
+    oracle for the plain cycles and the PCG."""
+    import qsm_gb300._lib as _lib
+    import qsm_gb300.synthetic as S
+
+    f, m, _ = S.poisson_case(shape, 41 + nl, semi=(0.3 * min(shape), 0.47 * min(shape)))
+    f = np.asfortranarray(f.astype(dt))
+    v0 = np.zeros(shape, order="F", dtype=dt)
+    L = _lib.lib()
+    assert L.qsm_ctx_set_debug(gpu_ctx.handle, 8) == 0
+    try:
+        gi = {}
+        a = qsm.mg_mex(v0, f, m, [1, 1, 1], -1.0, 1, 1, 2, 2, 2, nl, info=gi, ctx=gpu_ctx)
+        c = qsm.mgpcg_mex(v0, f, m, [1, 1, 1], 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl, ctx=gpu_ctx)
+    finally:
+        assert L.qsm_ctx_set_debug(gpu_ctx.handle, 0) == 0
+    assert gi["coarse_solver"] == solver
+    b = port.mg_mex(v0, f, m, [1, 1, 1], -1.0, 1, 1, 2, 2, 2, nl)
+    assert bits_equal(a, b), first_diff(a, b)
+    b = port.mgpcg_mex(v0, f, m, [1, 1, 1], 1e-6, 2, -1.0, 1, 1, 2, 2, 2, nl)
+    assert bits_equal(c, b), first_diff(c, b)
