@@ -761,10 +761,13 @@ qsm_status qsm_nifti_decode(qsm_ctx *ctx, const qsm_nifti_hdr *h, const void *pa
             copy_k<8><<<g, blk, 0, ctx->stream>>>((unsigned long long *)so.dev, (const unsigned long long *)in, o);
             break;
         }
-    } else if (h->scaled && (eb <= 2 || sdt == 16) && to_single && single_factors(h->scl_slope, h->scl_inter)) {
+    } else if (h->scaled && (eb <= 2 || sdt == 16) && to_single && single_factors(h->scl_slope, h->scl_inter) &&
+               !(eb == 1 && out_datatype == 64 && o.total >= 12000000)) {
         // a 224 x 224 x 128 x 4 int16 series (154 MB): the whole call 75 us, against 158
         // through the table, whose gathers cost an L1 access per voxel; single 224 x 224 x 128 x 2:
-        // at most 81 against 144 us in FP64 (the four-voxel form; one by one 143 and 93 us)
+        // at most 81 against 144 us in FP64 (the four-voxel form; one by one 143 and 93 us).
+        // 8 bits to double, one by one, only below 12 M voxels: the table has 256 entries and its
+        // gathers stay in L1 (224 x 224 x 128: 65-75 us, 69-73 through the table; x 4: 127-138, 110-116)
         const int64_t quads = o.total / 4;
         const bool by4 = out_datatype != 64 && o.perm[0] == 0 && o.n[0] % 4 == 0 && quads < 0xffffffffll - 152 * 4096 &&
                          o.rows <= 0x7fffffff && (uintptr_t)in % (4 * eb) == 0 && (uintptr_t)so.dev % 16 == 0;

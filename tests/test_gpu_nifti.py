@@ -220,3 +220,14 @@ def test_scaling_time_does_not_depend_on_midway_values(qn, dt, inter):
     plain = best(0.25, -3.0) if dt == 2 else best(0.25, 0.0)
     ties = best(0.1, inter) if dt == 2 else best(0.25, inter)
     assert ties < 2 * plain, (ties, plain)
+
+
+@pytest.mark.parametrize("slope", [0.1, 1e-30])
+def test_large_8_bit_image_to_double(qn, nio, slope):
+    """8-bit images of 12 M voxels or more to double go through the table of their
+    256 results, as images with factors outside the singles' range do."""
+    x = np.random.default_rng(6).integers(0, 256, (240, 220, 230), dtype=np.uint8)
+    hb = build_header("<", datatype=2, dim=(3, 240, 220, 230, 1, 1, 1, 1), slope=slope, inter=-0.3)
+    want = (np.float64(np.float32(slope)) * x + np.float64(np.float32(-0.3))).astype(np.float32).astype(np.float64)
+    img, _ = qn.decode(hb, x.tobytes(order="F"), out_dtype=np.float64)
+    assert np.array_equal(img, want)
