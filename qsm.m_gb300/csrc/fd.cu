@@ -261,6 +261,24 @@ __device__ __forceinline__ T wrap_pi(T x)
 // and more with six differences per voxel and tests on the FP64 pipe.
 constexpr int LAPW_R = 4, LAPW_TY = 4;
 
+// One voxel per thread, six wraps each: the form for volumes that do not fill the GPU
+// with columns, where a column's chain is the time.  Below the line of lapw_small, kernel
+// and launch in us over those of 3 x 3 x 3, voxels against columns: FP32 2 / 7 (33 x 31 x 29),
+// 1 / 8 (64 x 64 x 40), 9 / 11 (96^3), 13 / 17 (128 x 128 x 80), above 19.8 / 19.2 (128^3), 33 / 32
+// (181 x 217 x 91); FP64 10 / 17 (33 x 31 x 29), 19 / 20 (48^3), above 21 / 19 (64 x 64 x 40),
+// 398 / 271 (181 x 217 x 91).
+template <typename T> constexpr size_t lapw_small() { return sizeof(T) == 4 ? 2000000 : 130000; }
+template <typename T>
+__global__ void lapw_voxel_k(T *du, const T *__restrict__ u, H3<T> h, Dims d)
+{
+    VOXEL_PROLOGUE
+    if (i == 0 || j == 0 || k == 0 || i + 1 >= nx || j + 1 >= ny || k + 1 >= nz) return;
+    T v = h.x.w * (wrap_pi(u[l + 1] - u[l]) - wrap_pi(u[l] - u[l - 1]));
+    v = v + h.y.w * (wrap_pi(u[l + nx] - u[l]) - wrap_pi(u[l] - u[l - nx]));
+    v = v + h.z.w * (wrap_pi(u[l + nxny] - u[l]) - wrap_pi(u[l] - u[l - nxny]));
+    du[l] = v;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(32 * LAPW_TY) lapw_k(T *du, const T *__restrict__ u, H3<T> h, Dims d, int kz)
 {
@@ -347,6 +365,10 @@ static qsm_status launch_fd(qsm_ctx *ctx, FdOp op, const Dims &d, void **a, cons
     case OP_LAP1: lap1_k<T><<<g, b, 0, s>>>(o0, (const T *)a[1], G, inv_h2<T>(h), d); break;
     case OP_LAPW: {
         if (d.nx < 3 || d.ny < 3 || d.nz < 3) break;
+        if (d.n() < lapw_small<T>()) {
+            lapw_voxel_k<T><<<g, b, 0, s>>>(o0, (const T *)a[1], inv_h2<T>(h), d);
+            break;
+        }
         // columns of 16 planes; shorter ones where those would leave SMs without a few blocks each
         const unsigned gx = (unsigned)((d.nx - 2 + 30) / 31), gy = (unsigned)((d.ny - 2 + LAPW_R * LAPW_TY - 1) / (LAPW_R * LAPW_TY));
         int kz = 16;

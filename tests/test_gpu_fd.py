@@ -117,6 +117,21 @@ def test_fd_errors(gpu_ctx, qsm):
         qsm.gradf_mex(b, b.copy(order="F"), b.copy(order="F"), np.zeros((4, 4, 4), order="F"), [1, 1, 1])
 
 
+@pytest.mark.parametrize("dt,shape", [("float32", (130, 125, 127)), ("float32", (63, 4, 8001)), ("float32", (3, 700, 960)),
+                                      ("float32", (125, 127, 125)), ("float64", (33, 19, 220)), ("float64", (96, 35, 41)),
+                                      ("float64", (3, 209, 210)), ("float64", (65, 48, 41))])
+def test_lapw_both_forms_vs_oracle(gpu_ctx, qsm, port, dt, shape):
+    """The wrapped Laplacian in columns (from 2 M voxels in FP32, 130 k in FP64) and
+    one voxel per thread (the fourth and the last case lie just below): tile edges,
+    thin volumes, several turns.  Bit-for-bit against the oracle."""
+    u = np.asfortranarray((np.random.default_rng(sum(shape)).standard_normal(shape) * 6).astype(dt))
+    u[::7] *= 40
+    a, b = np.full(shape, 7.0, dt, order="F"), np.full(shape, 7.0, dt, order="F")
+    qsm.lapw_mex(a, u, [0.7, 1.0, 1.3])
+    port.lapw_mex(b, u, [0.7, 1.0, 1.3])
+    assert bits_equal(a, b), first_diff(a, b)
+
+
 @pytest.mark.parametrize("shape", [(3, 3, 3), (32, 5, 4), (33, 19, 20), (34, 18, 3), (65, 6, 37), (96, 35, 18)])
 @pytest.mark.parametrize("dt", ("float64", "float32"))
 def test_lapw_tiles_and_wraps_vs_oracle(gpu_ctx, qsm, port, shape, dt):
