@@ -59,17 +59,15 @@ PrimalC<T> make_primal_c(double tau, const double *h)
     return c;
 }
 
-template <typename T>
-static DualK<T> dual_k(const DualC<T> &c)
+static DualK dual_k(const DualC<double> &c)
 {
-    return DualK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.hx2), make_kmul(c.hy2), make_kmul(c.hz2),
+    return DualK{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.hx2), make_kmul(c.hy2), make_kmul(c.hz2),
                     make_kmul(c.lhx), make_kmul(c.lhy), make_kmul(c.lhz), make_kmul(c.lhh), make_kmul(c.whx), make_kmul(c.why),
                     make_kmul(c.whz), make_kmul(c.whh), make_kmul(c.alp0), make_kmul(c.alp1), make_kmul(c.sg), c.alp02, c.alp12};
 }
-template <typename T>
-static PrimalK<T> primal_k(const PrimalC<T> &c)
+static PrimalK primal_k(const PrimalC<double> &c)
 {
-    return PrimalK<T>{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.lhx), make_kmul(c.lhy), make_kmul(c.lhz),
+    return PrimalK{make_kmul(c.hx), make_kmul(c.hy), make_kmul(c.hz), make_kmul(c.lhx), make_kmul(c.lhy), make_kmul(c.lhz),
                       make_kmul(c.lhh), make_kmul(c.whx), make_kmul(c.why), make_kmul(c.whz), make_kmul(c.whh), make_kmul(c.tt),
                       make_kmul(c.tau1)};
 }
@@ -166,9 +164,15 @@ static inline dim3 interior_grid(const Dims &d)
     return vox_grid(e);
 }
 
+// Products of two variables and c / sqrt(x), on the pipes of the constants' kind
+// (plain ones: hardware instructions).
+template <typename T> __device__ __forceinline__ T pmul(const DualC<T> &, T a, T b) { return a * b; }
+__device__ __forceinline__ double pmul(const DualK &, double a, double b) { return xmul(a, b); }
+template <typename T> __device__ __forceinline__ T over_sqrt(T c, T x) { return c / sqrt(x); }
+
 // update_dual{d,f} of pd_tgv_mex.c:332-646.
-template <typename T>
-__device__ __forceinline__ void tgv_dual(const PdState<T> &s, const DualK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
+template <typename T, typename C>
+__device__ __forceinline__ void tgv_dual(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
     const T *chi_ = s.chi_, *eta_ = s.eta_;
     const T *w1 = s.w_, *w2 = s.w_ + N, *w3 = s.w_ + 2 * N;
@@ -184,10 +188,10 @@ __device__ __forceinline__ void tgv_dual(const PdState<T> &s, const DualK<T> &c,
     T a1 = p1[l] + c.hx * (chi_[l + 1] - c0) - c.sg * w1[l];
     T a2 = p2[l] + c.hy * (chi_[l + nx] - c0) - c.sg * w2[l];
     T a3 = p3[l] + c.hz * (chi_[l + nxny] - c0) - c.sg * w3[l];
-    T x = xmul(a1, a1) + xmul(a2, a2) + xmul(a3, a3);
+    T x = pmul(c, a1, a1) + pmul(c, a2, a2) + pmul(c, a3, a3);
     if (above(x, c.alp12)) {
         x = over_sqrt(c.alp1, x);
-        a1 = xmul(a1, x); a2 = xmul(a2, x); a3 = xmul(a3, x);
+        a1 = pmul(c, a1, x); a2 = pmul(c, a2, x); a3 = pmul(c, a3, x);
     }
     p1[l] = a1; p2[l] = a2; p3[l] = a3;
 
@@ -198,17 +202,17 @@ __device__ __forceinline__ void tgv_dual(const PdState<T> &s, const DualK<T> &c,
     T b4 = q4[l] + c.hy * (w2[l + nx] - v2);
     T b5 = q5[l] + c.hy2 * (w3[l + nx] - v3) + c.hz2 * (w2[l + nxny] - v2);
     T b6 = q6[l] + c.hz * (w3[l + nxny] - v3);
-    x = xmul(b1, b1) + xmul(b4, b4) + xmul(b6, b6) + scale2<1>(xmul(b2, b2) + xmul(b3, b3) + xmul(b5, b5));
+    x = pmul(c, b1, b1) + pmul(c, b4, b4) + pmul(c, b6, b6) + scale2<1>(pmul(c, b2, b2) + pmul(c, b3, b3) + pmul(c, b5, b5));
     if (above(x, c.alp02)) {
         x = over_sqrt(c.alp0, x);
-        b1 = xmul(b1, x); b2 = xmul(b2, x); b3 = xmul(b3, x); b4 = xmul(b4, x); b5 = xmul(b5, x); b6 = xmul(b6, x);
+        b1 = pmul(c, b1, x); b2 = pmul(c, b2, x); b3 = pmul(c, b3, x); b4 = pmul(c, b4, x); b5 = pmul(c, b5, x); b6 = pmul(c, b6, x);
     }
     q1[l] = b1; q2[l] = b2; q3[l] = b3; q4[l] = b4; q5[l] = b5; q6[l] = b6;
 }
 
 // update_primal{d,f} of pd_tgv_mex.c:659-977 (THETA = 1 extragradient).
-template <typename T>
-__device__ __forceinline__ void tgv_primal(const PdState<T> &s, const PrimalK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
+template <typename T, typename C>
+__device__ __forceinline__ void tgv_primal(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
     const T *nu = s.nu;
     const T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
@@ -233,8 +237,8 @@ __device__ __forceinline__ void tgv_primal(const PdState<T> &s, const PrimalK<T>
 }
 
 // update_dual{d,f} of pd_tv_mex.c:314-513.
-template <typename T>
-__device__ __forceinline__ void tv_dual(const PdState<T> &s, const DualK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
+template <typename T, typename C>
+__device__ __forceinline__ void tv_dual(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
     const T *chi_ = s.chi_, *eta_ = s.eta_;
     T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
@@ -247,17 +251,17 @@ __device__ __forceinline__ void tv_dual(const PdState<T> &s, const DualK<T> &c, 
     T a1 = p1[l] + c.hx * (chi_[l + 1] - c0);
     T a2 = p2[l] + c.hy * (chi_[l + nx] - c0);
     T a3 = p3[l] + c.hz * (chi_[l + nxny] - c0);
-    T x = xmul(a1, a1) + xmul(a2, a2) + xmul(a3, a3);
+    T x = pmul(c, a1, a1) + pmul(c, a2, a2) + pmul(c, a3, a3);
     if (above(x, c.alp12)) {
         x = over_sqrt(c.alp1, x);
-        a1 = xmul(a1, x); a2 = xmul(a2, x); a3 = xmul(a3, x);
+        a1 = pmul(c, a1, x); a2 = pmul(c, a2, x); a3 = pmul(c, a3, x);
     }
     p1[l] = a1; p2[l] = a2; p3[l] = a3;
 }
 
 // update_primal{d,f} of pd_tv_mex.c:524-727.
-template <typename T>
-__device__ __forceinline__ void tv_primal(const PdState<T> &s, const PrimalK<T> &c, size_t nx, size_t nxny, size_t N, size_t l)
+template <typename T, typename C>
+__device__ __forceinline__ void tv_primal(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
     const T *nu = s.nu;
     const T *p1 = s.p, *p2 = s.p + N, *p3 = s.p + 2 * N;
@@ -276,15 +280,15 @@ __device__ __forceinline__ void tv_primal(const PdState<T> &s, const PrimalK<T> 
 // The two updates of an iteration as kernels: over the interior of the grid, or
 // over the list of its voxels in the mask (FP64: an FP64 instruction takes its
 // slot in the pipe whatever lanes are active, and a row of the grid leaves a
-// third of them off at the mask's edge).
+// third of them off at the mask's edge), with products on the integer pipes.
 enum { PD_TGV_DUAL, PD_TGV_PRIMAL, PD_TV_DUAL, PD_TV_PRIMAL };
 template <int STEP, typename T, typename C>
 __device__ __forceinline__ void pd_step(const PdState<T> &s, const C &c, size_t nx, size_t nxny, size_t N, size_t l)
 {
-    if constexpr (STEP == PD_TGV_DUAL) tgv_dual<T>(s, c, nx, nxny, N, l);
-    if constexpr (STEP == PD_TGV_PRIMAL) tgv_primal<T>(s, c, nx, nxny, N, l);
-    if constexpr (STEP == PD_TV_DUAL) tv_dual<T>(s, c, nx, nxny, N, l);
-    if constexpr (STEP == PD_TV_PRIMAL) tv_primal<T>(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TGV_DUAL) tgv_dual(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TGV_PRIMAL) tgv_primal(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TV_DUAL) tv_dual(s, c, nx, nxny, N, l);
+    if constexpr (STEP == PD_TV_PRIMAL) tv_primal(s, c, nx, nxny, N, l);
 }
 
 template <int STEP, typename T, typename C>
@@ -336,6 +340,18 @@ __global__ void pd_seg_k(PdLists out, unsigned *seg, const uint8_t *__restrict__
     }
 }
 
+// Whether a FP64 solve takes the lists: not where the grid leaves SMs idle, whose time is the
+// chain of one thread and longer on the integer pipes (us an iteration, grid against
+// lists, TGV / TV on an ellipsoid: 33 x 31 x 29 25.0 / 18.8, 27.0 / 20.9; 36^3 37.1 / 24.8, 28.9 / 20.8;
+// 64^3 78.5 / 51.8, 36.4 / 24.3), nor where the iterations do not repay making them
+// (~70 us: TV at 36^3 after 17 iterations, at 48^3 after 5, at 64^3 after 3).
+static bool pd_use_lists(const Dims &d, uint32_t maxiter)
+{
+    if (d.nx < 3 || d.ny < 3 || d.nz < 3) return false;
+    const size_t n = (d.nx - 2) * (d.ny - 2) * (d.nz - 2);
+    return n >= 30000 && n * maxiter >= 700000;
+}
+
 // Builds the lists into *blk (left null where they are not used: FP32, whose
 // kernels HBM bounds, or no memory for them).
 static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t *mi, const uint8_t *m, PdLists *out, void **blk)
@@ -373,14 +389,14 @@ static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t 
     return dfree(ctx, seg);
 }
 
-template <int STEP, typename T, typename C>
-static void launch_step(qsm_ctx *ctx, const PdState<T> &s, const C &c, const Dims &d, const PdLists &ls, bool lists,
+template <int STEP, typename T, typename C, typename K>
+static void launch_step(qsm_ctx *ctx, const PdState<T> &s, const C &c, const K &ck, const Dims &d, const PdLists &ls, bool lists,
                         const PdCtl *ctl)
 {
     const int q = STEP == PD_TGV_DUAL || STEP == PD_TV_DUAL ? 0 : 1;
     if constexpr (sizeof(T) == 8) {
         if (lists) {
-            if (ls.n[q]) pd_list_k<STEP, T, C><<<(ls.n[q] + 255) / 256, 256, 0, ctx->stream>>>(s, c, d, ls.l[q], ls.n[q], ctl);
+            if (ls.n[q]) pd_list_k<STEP, T, K><<<(ls.n[q] + 255) / 256, 256, 0, ctx->stream>>>(s, ck, d, ls.l[q], ls.n[q], ctl);
             return;
         }
     }
@@ -496,13 +512,19 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
     const double alpha1 = lam, alpha0 = alpha * lam;
     QSM_TRY(launch_masks(ctx, s.m, s.mi, mask_dev, d));
     QSM_TRY((launch_scale<T, T>(ctx, s.f, (const T *)d2f_dev, sigma, N)));
-    const DualK<T> dc = dual_k(tgv ? make_dual_c<T>(sigma, h, alpha0, alpha1) : make_dual_c<T>(sigma, h, 0.0, lam));
-    const PrimalK<T> pc = primal_k(make_primal_c<T>(tau, h));
+    const DualC<T> dc = tgv ? make_dual_c<T>(sigma, h, alpha0, alpha1) : make_dual_c<T>(sigma, h, 0.0, lam);
+    const PrimalC<T> pc = make_primal_c<T>(tau, h);
+    DualK dk{};
+    PrimalK pk{};
+    if constexpr (sizeof(T) == 8) {
+        dk = dual_k(dc);
+        pk = primal_k(pc);
+    }
     const dim3 g = interior_grid(d);
     const bool empty = g.x == 0 || g.y == 0 || g.z == 0;
     PdLists ls;
     void *lblk = nullptr;
-    QSM_TRY(pd_lists(ctx, sizeof(T) == 8, d, s.mi, s.m, &ls, &lblk));
+    QSM_TRY(pd_lists(ctx, sizeof(T) == 8 && pd_use_lists(d, maxiter), d, s.mi, s.m, &ls, &lblk));
 
     cudaEvent_t e0, e1;
     QSM_CUDA(cudaEventCreate(&e0));
@@ -521,11 +543,11 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
         }
         if (!empty) {
             if (tgv) {
-                launch_step<PD_TGV_DUAL>(ctx, s, dc, d, ls, lblk != nullptr, ctl);
-                launch_step<PD_TGV_PRIMAL>(ctx, s, pc, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TGV_DUAL>(ctx, s, dc, dk, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TGV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk != nullptr, ctl);
             } else {
-                launch_step<PD_TV_DUAL>(ctx, s, dc, d, ls, lblk != nullptr, ctl);
-                launch_step<PD_TV_PRIMAL>(ctx, s, pc, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TV_DUAL>(ctx, s, dc, dk, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk != nullptr, ctl);
             }
             QSM_CUDA(cudaGetLastError());
         }

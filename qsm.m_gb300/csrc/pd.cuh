@@ -38,16 +38,14 @@ struct PrimalC {
     T hx, hy, hz, lhx, lhy, lhz, lhh, whx, why, whz, whh, tt, tau1;
 };
 
-// The same constants as factors of the plain path's kernels, which in FP64 the
-// FP64 pipe bounds: products run on the integer pipes (fp64.cuh).
-template <typename T>
+// The same constants as factors of the plain path's FP64 kernels where the FP64 pipe
+// bounds them: products run on the integer pipes (fp64.cuh).
 struct DualK {
-    KMul<T> hx, hy, hz, hx2, hy2, hz2, lhx, lhy, lhz, lhh, whx, why, whz, whh, alp0, alp1, sg;
-    T alp02, alp12;
+    KMul<double> hx, hy, hz, hx2, hy2, hz2, lhx, lhy, lhz, lhh, whx, why, whz, whh, alp0, alp1, sg;
+    double alp02, alp12;
 };
-template <typename T>
 struct PrimalK {
-    KMul<T> hx, hy, hz, lhx, lhy, lhz, lhh, whx, why, whz, whh, tt, tau1;
+    KMul<double> hx, hy, hz, lhx, lhy, lhz, lhh, whx, why, whz, whh, tt, tau1;
 };
 
 void pd_steps(const double *h, double *tau, double *sigma);

@@ -292,3 +292,29 @@ def test_pd_plain_voxel_lists(gpu_ctx, qsm, port, shape, kind):
     a = qsm.pd_tv_mex(f, m, h, 0.003, 0.0, 23)
     b = port.pd_tv_mex(f, m, h, 0.003, 0.0, 23)
     assert bits_equal(a, b), first_diff(a, b)
+
+
+@pytest.mark.parametrize("shape,iters,kind", [((33, 31, 29), 60, "dots"), ((36, 36, 36), 17, "dots"), ((36, 36, 36), 18, "dots"),
+                                              ((38, 29, 32), 40, "full"), ((38, 30, 32), 40, "full"), ((67, 9, 70), 28, "faces"),
+                                              ((34, 35, 33), 23, "none"), ((3, 99, 330), 23, "full"), ((65, 40, 19), 30, "ball")])
+@pytest.mark.parametrize("tgv", [True, False])
+def test_pd_plain_both_forms_fp64(gpu_ctx, qsm, port, shape, iters, kind, tgv):
+    """The plain FP64 path over the grid with hardware products, and over voxel lists
+    with integer ones (from 30000 interior voxels and 700000 voxel iterations): sizes and
+    iteration counts on both sides of each line, masks as above.  Bit-for-bit
+    against the oracle."""
+    rng = np.random.default_rng(sum(shape) + iters)
+    i, j, k = np.ogrid[0:shape[0], 0:shape[1], 0:shape[2]]
+    m = {"full": np.ones(shape, bool), "dots": rng.random(shape) < 0.8, "none": np.zeros(shape, bool),
+         "faces": (i < 2) | (j == shape[1] - 1) | (k < 3) | (i > shape[0] - 3),
+         "ball": sum(((a - (n - 1) / 2) / (0.45 * n)) ** 2 for a, n in zip((i, j, k), shape)) <= 1}[kind]
+    m = np.asfortranarray(np.broadcast_to(m, shape).astype(np.uint8))
+    f = np.asfortranarray(rng.standard_normal(shape) * 0.3)
+    h = [1.0, 0.9, 1.3]
+    if tgv:
+        a = qsm.pd_tgv_mex(f, m, h, 2e-3, 2.0, 1e-12, iters)
+        b = port.pd_tgv_mex(f, m, h, 2e-3, 2.0, 1e-12, iters)
+    else:
+        a = qsm.pd_tv_mex(f, m, h, 2e-3, 1e-12, iters)
+        b = port.pd_tv_mex(f, m, h, 2e-3, 1e-12, iters)
+    assert bits_equal(a, b), first_diff(a, b)
