@@ -443,6 +443,42 @@ FusedArgs pd_volume_args(const PdVolume &v, int var, uint32_t it)
     return s;
 }
 
+namespace {
+struct TuneRun {
+    int var;
+    float ms;
+};
+bool faster(const TuneRun &a, const TuneRun &b) { return a.ms < b.ms; }
+}  // namespace
+
+// Times n iterations of each run, queued one after another (one more first, untimed).
+static qsm_status tune_time(qsm_ctx *ctx, const PdVolume &v, std::vector<TuneRun> &runs, uint32_t n)
+{
+    std::vector<cudaEvent_t> ev(2 * runs.size(), nullptr);
+    const auto body = [&]() -> qsm_status {
+        for (cudaEvent_t &e : ev) QSM_CUDA(cudaEventCreate(&e));
+        for (size_t r = 0; r < runs.size(); ++r) {
+            const int k = runs[r].var;
+            for (uint32_t it = 0; it <= n; ++it) {
+                if (it == 1) QSM_CUDA(cudaEventRecord(ev[2 * r], ctx->stream));
+                QSM_TRY(launch_variant(ctx, ctx->stream, k, v.tgv, false, v.tl[k].nact, pd_volume_args(v, k, it), v.dc, v.pc,
+                                       v.d, 0.0, it + 1, volume_maps(v, k, it), it > 0));
+            }
+            QSM_CUDA(cudaEventRecord(ev[2 * r + 1], ctx->stream));
+        }
+        QSM_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (size_t r = 0; r < runs.size(); ++r) {
+            QSM_CUDA(cudaEventElapsedTime(&runs[r].ms, ev[2 * r], ev[2 * r + 1]));
+            runs[r].ms /= (float)n;
+        }
+        return QSM_OK;
+    };
+    const qsm_status st = body();
+    for (cudaEvent_t e : ev)
+        if (e) cudaEventDestroy(e);
+    return st;
+}
+
 qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
 {
     Range nvtx_range("pd_fused/autotune");
@@ -465,38 +501,28 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
     v->var = 0;
     QSM_TRY(pd_volume_tiles(ctx, v, 0));
     if (v->tl[0].nact == 0 || maxiter < 20) return QSM_OK;
-    // time each variant over a few iterations on this problem, then reset the state
-    cudaEvent_t t0, t1;
-    QSM_CUDA(cudaEventCreate(&t0));
-    QSM_CUDA(cudaEventCreate(&t1));
-    float best = 1e30f;
-    for (int k = 0; k < kNumVariants; ++k) {
-        if (!variant_ok(*v, k)) continue;
-        QSM_TRY(pd_volume_tiles(ctx, v, k));
-        for (uint32_t it = 0; it < 2; ++it)
-            QSM_TRY(launch_variant(ctx, ctx->stream, k, v->tgv, false, v->tl[k].nact, pd_volume_args(*v, k, it),
-                                   v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it), it > 0));
-        // six iterations, then, where those take under 0.3 ms, 36 more
-        float ms = 0.f;
-        for (uint32_t i0 = 2, n = 6;; n = 36) {
-            QSM_CUDA(cudaEventRecord(t0, ctx->stream));
-            for (uint32_t it = i0; it < i0 + n; ++it)
-                QSM_TRY(launch_variant(ctx, ctx->stream, k, v->tgv, false, v->tl[k].nact, pd_volume_args(*v, k, it),
-                                       v->dc, v->pc, v->d, 0.0, it + 1, volume_maps(*v, k, it), true));
-            QSM_CUDA(cudaEventRecord(t1, ctx->stream));
-            QSM_CUDA(cudaEventSynchronize(t1));
-            cudaEventElapsedTime(&ms, t0, t1);
-            ms /= (float)n;
-            i0 += n;
-            if (n != 6 || 6 * ms >= 0.3f) break;
-        }
-        if (ms < best) {
-            best = ms;
-            v->var = k;
-        }
+    // Timed on this problem, in a state whose duals are all projected (most are, later in a
+    // solve), then the state is reset: two iterations of each variant; eight (four above
+    // 20 us) of those within a fifth of the best; 24 more of those within 3 % where the
+    // solve is long enough to repay them.  (A new size
+    // costs 48^3 TGV 2.1 ms; eight iterations of every variant 3.5, 44 of them 14.)
+    for (int k = 0; k < kNumVariants; ++k)
+        if (variant_ok(*v, k)) QSM_TRY(pd_volume_tiles(ctx, v, k));
+    std::vector<TuneRun> runs;
+    for (int k = 0; k < kNumVariants; ++k)
+        if (variant_ok(*v, k)) runs.push_back({k, 0.f});
+    QSM_CUDA(cudaMemsetAsync(v->PA[0], 0x3f, v->state_bytes, ctx->stream));
+    float best = 0.f;
+    for (int phase = 0;; ++phase) {
+        QSM_TRY(tune_time(ctx, *v, runs, phase == 0 ? 2 : phase == 1 ? (best > 0.02f ? 4 : 8) : 24));
+        best = std::min_element(runs.begin(), runs.end(), faster)->ms;
+        std::vector<TuneRun> next;
+        for (const TuneRun &r : runs)
+            if (r.ms <= (phase == 0 ? 1.2f : 1.03f) * best) next.push_back(r);
+        if (phase == 2 || (phase == 1 && (next.size() == 1 || maxiter < 400))) break;
+        runs = next;
     }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
+    v->var = std::min_element(runs.begin(), runs.end(), faster)->var;
     QSM_CUDA(cudaMemsetAsync(v->PA[0], 0, v->state_bytes, ctx->stream));
     std::lock_guard<std::mutex> lock(g_tune_mu);
     tune_store_locked(key, v->var);
