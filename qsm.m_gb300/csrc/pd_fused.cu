@@ -219,7 +219,9 @@ static qsm_status set_all_smem(qsm_ctx *ctx)
     return stream_set_smem(ctx);
 }
 
-// process-wide tuning table: (tgv, nx, ny, nz) -> variant
+// process-wide tuning table: (tgv, nx, ny, nz) -> variant, plus TUNE_PLAIN where its
+// iterations are not chained
+constexpr int TUNE_PLAIN = 64;
 using TuneKey = std::tuple<int, size_t, size_t, size_t>;
 static std::map<TuneKey, int> g_tuned;
 static std::mutex g_tune_mu;
@@ -236,7 +238,7 @@ static void tune_load_locked()
     int tg, v;
     size_t a, b, c;
     while (fscanf(fp, "%d %zu %zu %zu %d", &tg, &a, &b, &c, &v) == 5)
-        if (v >= 0 && v < kNumVariants) g_tuned[TuneKey(tg, a, b, c)] = v;
+        if (v >= 0 && v < 2 * TUNE_PLAIN && (v & ~TUNE_PLAIN) < kNumVariants) g_tuned[TuneKey(tg, a, b, c)] = v;
     fclose(fp);
 }
 
@@ -446,10 +448,41 @@ FusedArgs pd_volume_args(const PdVolume &v, int var, uint32_t it)
 namespace {
 struct TuneRun {
     int var;
+    bool chain;
     float ms;
 };
 bool faster(const TuneRun &a, const TuneRun &b) { return a.ms < b.ms; }
 }  // namespace
+
+template <int TX, int TY, int TZ, int MINB>
+static const void *tile_kernel(bool tgv)
+{
+    return tgv ? (const void *)tgv_fused_k<TX, TY, TZ, MINB, false> : (const void *)tv_fused_k<TX, TY, TZ, MINB, false>;
+}
+
+// Whether variant var's iterations may be chained on this volume.  Chained CTAs of the next
+// iteration take the free places of an SM while this one runs, two and more on one SM while
+// others stay empty: harmless where an SM holds one, where the CTAs are few, and where they
+// nearly fill the GPU, but up to 22 % slower in between (us an iteration chained / plain, by
+// CTAs of 304: 30 10.9 / 12.9, 77 13.5 / 13.5, 136 15.2 / 13.8, 184 14.1 / 13.7, 216 15.9 / 17.8;
+// of 608: 54 11.3 / 13.5, 236 17.6 / 14.4, 400 18.3 / 17.7, 578 20.4 / 21.8), and not within the few
+// iterations of a timed run.  TV's tiles of two planes gain throughout (8.6-10.6 / 11.2).
+static bool chain_ok(qsm_ctx *ctx, const PdVolume &v, int var)
+{
+    const Variant &x = kVariants[var];
+    const void *k = x.stream ? stream_kernel(x.tx, x.ty, v.tgv, x.tma)
+                  : var == 0 ? tile_kernel<32, 8, 4, 4>(v.tgv) : var == 1 ? tile_kernel<32, 8, 2, 4>(v.tgv)
+                  : var == 2 ? tile_kernel<32, 4, 4, 8>(v.tgv) : tile_kernel<32, 16, 2, 2>(v.tgv);
+    int occ = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, variant_threads(var), variant_smem(var, v.tgv)) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const unsigned nact = v.tl[var].nact;
+    if (!v.tgv && !x.stream && x.tz == 2) return true;
+    return occ == 1 || nact <= (unsigned)sms / (x.stream ? 4 : 2) || nact >= 7u * (unsigned)(occ * sms) / 10;
+}
 
 // Times n iterations of each run, queued one after another (one more first, untimed).
 static qsm_status tune_time(qsm_ctx *ctx, const PdVolume &v, std::vector<TuneRun> &runs, uint32_t n)
@@ -462,7 +495,7 @@ static qsm_status tune_time(qsm_ctx *ctx, const PdVolume &v, std::vector<TuneRun
             for (uint32_t it = 0; it <= n; ++it) {
                 if (it == 1) QSM_CUDA(cudaEventRecord(ev[2 * r], ctx->stream));
                 QSM_TRY(launch_variant(ctx, ctx->stream, k, v.tgv, false, v.tl[k].nact, pd_volume_args(v, k, it), v.dc, v.pc,
-                                       v.d, 0.0, it + 1, volume_maps(v, k, it), it > 0));
+                                       v.d, 0.0, it + 1, volume_maps(v, k, it), runs[r].chain && it > 0));
             }
             QSM_CUDA(cudaEventRecord(ev[2 * r + 1], ctx->stream));
         }
@@ -493,8 +526,9 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
         std::lock_guard<std::mutex> lock(g_tune_mu);
         tune_load_locked();
         auto itk = g_tuned.find(key);
-        if (itk != g_tuned.end() && variant_ok(*v, itk->second)) {
-            v->var = itk->second;
+        if (itk != g_tuned.end() && variant_ok(*v, itk->second & ~TUNE_PLAIN)) {
+            v->var = itk->second & ~TUNE_PLAIN;
+            v->chain = !(itk->second & TUNE_PLAIN);
             return pd_volume_tiles(ctx, v, v->var);
         }
     }
@@ -503,14 +537,14 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
     if (v->tl[0].nact == 0 || maxiter < 20) return QSM_OK;
     // Timed on this problem, in a state whose duals are all projected (most are, later in a
     // solve), then the state is reset: two iterations of each variant; eight (four above
-    // 20 us) of those within a fifth of the best; 24 more of those within 3 % where the
-    // solve is long enough to repay them.  (A new size
+    // 20 us) of those within a fifth of the best, plain and, where that may be, chained; 24
+    // more of those within 3 % where the solve is long enough to repay them.  (A new size
     // costs 48^3 TGV 2.1 ms; eight iterations of every variant 3.5, 44 of them 14.)
     for (int k = 0; k < kNumVariants; ++k)
         if (variant_ok(*v, k)) QSM_TRY(pd_volume_tiles(ctx, v, k));
     std::vector<TuneRun> runs;
     for (int k = 0; k < kNumVariants; ++k)
-        if (variant_ok(*v, k)) runs.push_back({k, 0.f});
+        if (variant_ok(*v, k)) runs.push_back({k, false, 0.f});
     QSM_CUDA(cudaMemsetAsync(v->PA[0], 0x3f, v->state_bytes, ctx->stream));
     float best = 0.f;
     for (int phase = 0;; ++phase) {
@@ -518,14 +552,19 @@ qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter)
         best = std::min_element(runs.begin(), runs.end(), faster)->ms;
         std::vector<TuneRun> next;
         for (const TuneRun &r : runs)
-            if (r.ms <= (phase == 0 ? 1.2f : 1.03f) * best) next.push_back(r);
+            if (r.ms <= (phase == 0 ? 1.2f : 1.03f) * best) {
+                next.push_back(r);
+                if (phase == 0 && chain_ok(ctx, *v, r.var)) next.push_back({r.var, true, 0.f});
+            }
         if (phase == 2 || (phase == 1 && (next.size() == 1 || maxiter < 400))) break;
         runs = next;
     }
-    v->var = std::min_element(runs.begin(), runs.end(), faster)->var;
+    const TuneRun &r = *std::min_element(runs.begin(), runs.end(), faster);
+    v->var = r.var;
+    v->chain = r.chain;
     QSM_CUDA(cudaMemsetAsync(v->PA[0], 0, v->state_bytes, ctx->stream));
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    tune_store_locked(key, v->var);
+    tune_store_locked(key, v->var | (v->chain ? 0 : TUNE_PLAIN));
     return QSM_OK;
 }
 
@@ -593,7 +632,7 @@ qsm_status pd_fused(qsm_ctx *ctx, bool tgv, const Dims &d, qsm_dtype dt, const v
         const bool chk = ((it + 1) % 10) == 0;
         if (!empty)
             QSM_TRY(launch_variant(ctx, ctx->stream, var, tgv, chk, nact, pd_volume_args(v, var, it), v.dc, v.pc, d,
-                                   tol, it + 1, volume_maps(v, var, it), it > 0));
+                                   tol, it + 1, volume_maps(v, var, it), it > 0 && v.chain));
         enq = it + 1;
         const bool print = verbose && (it == 0 || it == maxiter - 1 || ((it + 1) % pmod) == 0);
         if (print || (chk && ((it + 1) % 100) == 0)) {

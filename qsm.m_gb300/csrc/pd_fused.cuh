@@ -213,6 +213,8 @@ struct TmaMaps {
 size_t stream_smem(int tx, int ty, bool tgv);
 size_t stream_tma_smem(int tx, int ty);
 qsm_status stream_set_smem(qsm_ctx *ctx);
+// the kernel stream_launch runs for these arguments (without the monitor), for occupancy queries; null: none
+const void *stream_kernel(int tx, int ty, bool tgv, bool tma);
 // tm: the TMA column kernel (TGV) with these maps; null: the register-prefetch one
 qsm_status stream_launch(qsm_ctx *ctx, cudaStream_t st, int tx, int ty, int cz, bool tgv, bool chk, unsigned nact,
                          const FusedArgs &s, const DualC<float> &dc, const PrimalC<float> &pc, const Dims &d,
@@ -266,6 +268,8 @@ struct PdVolume {
     DualC<float> dc{};
     PrimalC<float> pc{};
     int var = 0;                 // chosen tile variant
+    bool chain = true;           // whether a solve alone chains its iterations (sessions do: volumes of
+                                 // 40 x 36 x 34 to 70 x 40 x 52 together 2.9 ms a hundred, plain 3.4)
     // TMA maps per (variant, iterate rotation it % 3), filled for the TMA
     // variants; empty when they cannot run on this volume
     std::vector<TmaMaps> maps;
@@ -283,7 +287,7 @@ qsm_status pd_volume_init(qsm_ctx *ctx, PdVolume *v, bool tgv, const Dims &d, qs
 qsm_status pd_volume_tiles(qsm_ctx *ctx, PdVolume *v, int var);
 // Kernel arguments of variant var for the iteration that reads iterate `it`.
 FusedArgs pd_volume_args(const PdVolume &v, int var, uint32_t it);
-// Picks v->var: QSM_FUSED_VARIANT, the tuning table, or timing each variant
+// Picks v->var and v->chain: QSM_FUSED_VARIANT, the tuning table, or timing each variant
 // on this volume for a few iterations (the state is zeroed again after).
 qsm_status pd_volume_tune(qsm_ctx *ctx, PdVolume *v, uint32_t maxiter);
 // One iteration of variant v->var on stream st (the one-volume kernels); s

@@ -89,6 +89,13 @@ qsm_status stream_set_smem(qsm_ctx *ctx)
     return QSM_OK;
 }
 
+const void *stream_kernel(int, int ty, bool tgv, bool tma)
+{
+    if (tma) return ty == 16 ? (const void *)stream_tma_k<28, 16, false> : ty == 20 ? (const void *)stream_tma_k<28, 20, false> : (const void *)stream_tma_k<28, 24, false>;
+    if (ty == 12) return tgv ? (const void *)stream_k<28, 12, true, false> : (const void *)stream_k<28, 12, false, false>;
+    return tgv ? (const void *)stream_k<28, 16, true, false> : (const void *)stream_k<28, 16, false, false>;
+}
+
 template <int TX, int TY>
 static void launch_tma_t(cudaStream_t st, bool chain, bool chk, unsigned nact, const TmaMaps &tm, const FusedArgs &s,
                          const DualC<float> &dc, const PrimalC<float> &pc, const Dims &d, int cz, double tol,

@@ -345,3 +345,44 @@ def test_fused_first_solve_of_a_size_tunes_briefly(gpu_ctx, qsm):
     per = (min(solve(f, m, 540)[1] for _ in range(3)) - again) / 500
     assert first - again < 300 * per, (first, again, per)
     assert torch.equal(a, solve(f, m, 40)[0])
+
+
+def test_tuning_table_keeps_plain_iterations(gpu_ctx, qsm, tmp_path):
+    """The tuning file names a variant per size, plus 64 where its iterations are not
+    chained: both forms of one variant run and agree to the bit; lines that name no
+    variant are passed over."""
+    import os
+    import subprocess
+    import sys
+
+    cache = tmp_path / "tuned"
+    cache.write_text("1 44 42 40 1\n1 45 42 40 65\n0 45 42 40 66\n1 46 42 40 77\n1 47 42 40 200\n")
+    code = """
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import qsm_gb300 as qsm
+rng = np.random.default_rng(2)
+f = np.asfortranarray(rng.standard_normal((47, 42, 40)).astype(np.float32) * 0.05)
+m = np.asfortranarray((rng.random((47, 42, 40)) < 0.9).astype(np.uint8))
+m[43:] = 0
+def tgv(n):
+    info = {}
+    x = qsm.pd_tgv_mex(np.asfortranarray(f[:n]), np.asfortranarray(m[:n]), [1, 1, 1], 1e-3, 3.0, 1e-9, 50, fused=True, info=info)
+    return x[:43], info["tile"]
+chained, t0 = tgv(44)
+plain, t1 = tgv(45)
+assert t0 == t1 == (32, 8, 2), (t0, t1)
+assert np.array_equal(chained, plain)
+info = {}
+qsm.pd_tv_mex(np.asfortranarray(f[:45]), np.asfortranarray(m[:45]), [1, 1, 1], 1e-3, 1e-9, 20, fused=True, info=info)
+assert info["tile"] == (32, 4, 4), info
+for n in (46, 47):
+    assert np.array_equal(tgv(n)[0], chained)
+print("agree")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code, root], env={**os.environ, "QSM_AUTOTUNE_CACHE": str(cache)},
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "agree" in r.stdout, r.stdout + r.stderr
+    assert len(cache.read_text().splitlines()) == 7  # the two sizes without a valid line were tuned
