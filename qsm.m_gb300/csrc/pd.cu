@@ -340,6 +340,13 @@ __global__ void pd_seg_k(PdLists out, unsigned *seg, const uint8_t *__restrict__
     }
 }
 
+// A device block given back on every way out.
+struct PdBlock {
+    qsm_ctx *ctx;
+    void *p = nullptr;
+    ~PdBlock() { if (p) cudaFreeAsync(p, ctx->stream); }
+};
+
 // Whether a FP64 solve takes the lists: not where the grid leaves SMs idle, whose time is the
 // chain of one thread and longer on the integer pipes (us an iteration, grid against
 // lists, TGV / TV on an ellipsoid: 33 x 31 x 29 25.0 / 18.8, 27.0 / 20.9; 36^3 37.1 / 24.8, 28.9 / 20.8;
@@ -352,21 +359,20 @@ static bool pd_use_lists(const Dims &d, uint32_t maxiter)
     return n >= 30000 && n * maxiter >= 700000;
 }
 
-// Builds the lists into *blk (left null where they are not used: FP32, whose
+// Builds the lists into blk->p (left null where they are not used: FP32, whose
 // kernels HBM bounds, or no memory for them).
-static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t *mi, const uint8_t *m, PdLists *out, void **blk)
+static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t *mi, const uint8_t *m, PdLists *out, PdBlock *blk)
 {
-    *blk = nullptr;
     *out = PdLists{};
     const dim3 g = interior_grid(d);
     if (!use || g.x == 0 || g.y == 0 || g.z == 0 || d.n() >= ((size_t)1 << 31)) return QSM_OK;
     const size_t nseg = (size_t)g.x * (d.ny - 2) * (d.nz - 2);
-    void *seg = nullptr;
-    if (dalloc(ctx, &seg, (4 * nseg + scan_scratch(2 * nseg)) * sizeof(unsigned)) != QSM_OK) {
+    PdBlock seg{ctx};
+    if (dalloc(ctx, &seg.p, (4 * nseg + scan_scratch(2 * nseg)) * sizeof(unsigned)) != QSM_OK) {
         cudaGetLastError();
         return QSM_OK;
     }
-    unsigned *segc = (unsigned *)seg, *off = segc + 2 * nseg, *tmp = off + 2 * nseg;
+    unsigned *segc = (unsigned *)seg.p, *off = segc + 2 * nseg, *tmp = off + 2 * nseg;
     pd_seg_k<false><<<g, vox_block(), 0, ctx->stream>>>(PdLists{}, segc, mi, m, d, nseg);
     QSM_CUDA(cudaGetLastError());
     QSM_TRY(exclusive_scan(ctx, segc, off, 2 * nseg, tmp));
@@ -377,16 +383,15 @@ static qsm_status pd_lists(qsm_ctx *ctx, bool use, const Dims &d, const uint8_t 
     }
     QSM_CUDA(cudaStreamSynchronize(ctx->stream));
     const unsigned n0 = h[0] + h[2], n1 = h[1] + h[3] - n0;
-    if (dalloc(ctx, blk, ((size_t)n0 + n1 + 2) * sizeof(uint32_t)) != QSM_OK) {
+    if (dalloc(ctx, &blk->p, ((size_t)n0 + n1 + 2) * sizeof(uint32_t)) != QSM_OK) {
         cudaGetLastError();
-        *blk = nullptr;
-        return dfree(ctx, seg);
+        return QSM_OK;
     }
-    uint32_t *l = (uint32_t *)*blk;
+    uint32_t *l = (uint32_t *)blk->p;
     *out = PdLists{{l, l + n0}, {n0, n1}};
     pd_seg_k<true><<<g, vox_block(), 0, ctx->stream>>>(*out, off, mi, m, d, nseg);
     QSM_CUDA(cudaGetLastError());
-    return dfree(ctx, seg);
+    return QSM_OK;
 }
 
 template <int STEP, typename T, typename C, typename K>
@@ -489,10 +494,10 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
     Range nvtx_range("pd_plain");
     const size_t N = d.n();
     const int narr = tgv ? 23 : 11;
-    void *blk = nullptr;
-    QSM_TRY(dalloc(ctx, &blk, (size_t)narr * N * sizeof(T) + 2 * N + sizeof(PdCtl) + 256));
-    QSM_CUDA(cudaMemsetAsync(blk, 0, (size_t)narr * N * sizeof(T) + 2 * N + sizeof(PdCtl) + 256, ctx->stream));
-    T *b = (T *)blk;
+    PdBlock blk{ctx}, lblk{ctx};
+    QSM_TRY(dalloc(ctx, &blk.p, (size_t)narr * N * sizeof(T) + 2 * N + sizeof(PdCtl) + 256));
+    QSM_CUDA(cudaMemsetAsync(blk.p, 0, (size_t)narr * N * sizeof(T) + 2 * N + sizeof(PdCtl) + 256, ctx->stream));
+    T *b = (T *)blk.p;
     PdState<T> s;
     memset(&s, 0, sizeof s);
     if (tgv) {
@@ -523,13 +528,19 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
     const dim3 g = interior_grid(d);
     const bool empty = g.x == 0 || g.y == 0 || g.z == 0;
     PdLists ls;
-    void *lblk = nullptr;
     QSM_TRY(pd_lists(ctx, sizeof(T) == 8 && pd_use_lists(d, maxiter), d, s.mi, s.m, &ls, &lblk));
 
-    cudaEvent_t e0, e1;
-    QSM_CUDA(cudaEventCreate(&e0));
-    QSM_CUDA(cudaEventCreate(&e1));
-    QSM_CUDA(cudaEventRecord(e0, ctx->stream));
+    struct Events {
+        cudaEvent_t e[2] = {};
+        ~Events()
+        {
+            for (cudaEvent_t x : e)
+                if (x) cudaEventDestroy(x);
+        }
+    } ev;
+    QSM_CUDA(cudaEventCreate(&ev.e[0]));
+    QSM_CUDA(cudaEventCreate(&ev.e[1]));
+    QSM_CUDA(cudaEventRecord(ev.e[0], ctx->stream));
     const uint32_t pmod = maxiter ? maxiter / (verbose > 4 ? (verbose < maxiter ? verbose : maxiter) : (4 < maxiter ? 4 : maxiter)) : 1;
     if (verbose) printf("Iter\t\t||delta chi||\t||delta eta||\n");
     uint32_t enq = 0;
@@ -543,11 +554,11 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
         }
         if (!empty) {
             if (tgv) {
-                launch_step<PD_TGV_DUAL>(ctx, s, dc, dk, d, ls, lblk != nullptr, ctl);
-                launch_step<PD_TGV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TGV_DUAL>(ctx, s, dc, dk, d, ls, lblk.p != nullptr, ctl);
+                launch_step<PD_TGV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk.p != nullptr, ctl);
             } else {
-                launch_step<PD_TV_DUAL>(ctx, s, dc, dk, d, ls, lblk != nullptr, ctl);
-                launch_step<PD_TV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk != nullptr, ctl);
+                launch_step<PD_TV_DUAL>(ctx, s, dc, dk, d, ls, lblk.p != nullptr, ctl);
+                launch_step<PD_TV_PRIMAL>(ctx, s, pc, pk, d, ls, lblk.p != nullptr, ctl);
             }
             QSM_CUDA(cudaGetLastError());
         }
@@ -563,14 +574,12 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
             if (hctl.done) break;
         }
     }
-    QSM_CUDA(cudaEventRecord(e1, ctx->stream));
+    QSM_CUDA(cudaEventRecord(ev.e[1], ctx->stream));
     QSM_CUDA(cudaMemcpyAsync(&hctl, ctl, sizeof(PdCtl), cudaMemcpyDeviceToHost, ctx->stream));
     QSM_CUDA(cudaMemcpyAsync(chi_out, s.chi, N * sizeof(T), cudaMemcpyDeviceToDevice, ctx->stream));
     QSM_CUDA(cudaStreamSynchronize(ctx->stream));
     float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]);
     if (info) {
         info->iters = hctl.done ? hctl.iters : enq;
         info->monitor_chi = hctl.checks ? hctl.n1 : 1.0;
@@ -579,8 +588,6 @@ static qsm_status pd_plain(qsm_ctx *ctx, bool tgv, const Dims &d, const void *d2
         info->active_voxels = (uint64_t)(d.nx > 2 ? d.nx - 2 : 0) * (d.ny > 2 ? d.ny - 2 : 0) * (d.nz > 2 ? d.nz - 2 : 0);
         info->tile[0] = info->tile[1] = info->tile[2] = 0;
     }
-    if (lblk) QSM_TRY(dfree(ctx, lblk));
-    QSM_TRY(dfree(ctx, blk));
     return QSM_OK;
 }
 

@@ -386,3 +386,37 @@ print("agree")
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "agree" in r.stdout, r.stdout + r.stderr
     assert len(cache.read_text().splitlines()) == 7  # the two sizes without a valid line were tuned
+
+
+@pytest.mark.parametrize("tgv", [True, False])
+def test_plain_fp64_failure_keeps_no_memory(gpu_ctx, qsm, tgv):
+    """A plain FP64 solve that ends early with an error gives its device memory back.
+    The error is one that an earlier, refused call (a device number that does not
+    exist) left pending in the runtime, which the solve meets after its first launches."""
+    import ctypes
+
+    import qsm_gb300._lib as _lib
+
+    torch = pytest.importorskip("torch")
+    rt = ctypes.CDLL("libcudart.so.13")
+    f = torch.zeros((64, 64, 64), dtype=torch.float64, device="cuda")
+    m = torch.ones((64, 64, 64), dtype=torch.uint8, device="cuda")
+    out = torch.zeros_like(f)
+    dims, h = (ctypes.c_size_t * 3)(64, 64, 64), (ctypes.c_double * 3)(1, 1, 1)
+    pi = _lib.PdInfo()
+
+    def solve():
+        tail = (1e-9, 20, 0, ctypes.c_void_p(out.data_ptr()), ctypes.byref(pi))
+        head = (_lib.QSM_F64, dims, ctypes.c_void_p(f.data_ptr()), ctypes.c_void_p(m.data_ptr()), h, 1e-3)
+        gpu_ctx.call(*(("qsm_pd_tgv", *head, 3.0, *tail) if tgv else ("qsm_pd_tv", *head, *tail)))
+
+    solve()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for _ in range(40):
+        assert rt.cudaSetDevice(100000) != 0
+        with pytest.raises(qsm.QsmError):
+            solve()
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20  # (40 blocks of 23 or 11 arrays of 2 MiB)
+    solve()  # the context is as it was
