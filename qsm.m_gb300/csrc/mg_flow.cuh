@@ -27,7 +27,7 @@
 //
 // Bound by latency: a packet takes 700-1030 cycles from store to a successful
 // poll (measured alone), then five dependent FP64 operations of 64 cycles each
-// and the CTA's barrier; ~1.3 us a pass against 2.6 us with a barrier of the
+// and the CTA's barrier; 1.2-1.5 us a pass against 2.6 us with a barrier of the
 // grid.  Measured: see plan_coarse_grid.
 
 constexpr int FL_THREADS = 512;  // most threads of a CTA, one voxel of each colour per thread
