@@ -248,11 +248,23 @@ __device__ __forceinline__ float two_sum(float a, float b, float *err)
     *err = (a - (t - z)) + (b - z);
     return t;
 }
-__device__ __forceinline__ bool scale_range(float x) { return x == 0.0f || (fabsf(x) >= 0x1p-40f && fabsf(x) <= 0x1p60f); }
-template <bool INT>
-__device__ __forceinline__ float scale_single(float x, float slope, float inter, bool *sure)
+// The factors, and the stored singles (lo <= |x| <= hi, or 0) whose products with the
+// slope neither overflow nor have bits below 2^-149, so that pe is exact (others, and with
+// the bounds 2^-40 and 2^60 all of an image in units of 1e-14, take FP64: a call of
+// 224 x 224 x 128 x 2 singles 189 us instead of 64).
+struct ScaleF {
+    float slope, inter, lo, hi;
+};
+static ScaleF scale_factors(double slope, double inter)
 {
-    const float p = x * slope, pe = fmaf(x, slope, -p), y = fmaf(x, slope, inter);
+    const int e = std::ilogb(slope);
+    return ScaleF{(float)slope, (float)inter, std::ldexp(1.0f, std::max(-126, -103 - e)), std::ldexp(1.0f, std::min(127, 120 - e))};
+}
+__device__ __forceinline__ bool scale_range(float x, const ScaleF &c) { return x == 0.0f || (fabsf(x) >= c.lo && fabsf(x) <= c.hi); }
+template <bool INT>
+__device__ __forceinline__ float scale_single(float x, const ScaleF &c, bool *sure)
+{
+    const float slope = c.slope, inter = c.inter, p = x * slope, pe = fmaf(x, slope, -p), y = fmaf(x, slope, inter);
     float te;
     const float t = two_sum(p, inter, &te), e = ((t - y) + te) + pe;
     // half a unit on y's lower side (that of the single before y: a power of two has the
@@ -260,8 +272,7 @@ __device__ __forceinline__ float scale_single(float x, float slope, float inter,
     const uint32_t u = __float_as_uint(y) & 0x7fffffffu;
     const float half = __uint_as_float(((u - 1u) & 0x7f800000u) - (24u << 23));
     *sure = fabsf(e) * (1.0f + 1.0f / 32768.0f) < half;
-    // (outside this range of a stored single the error terms might underflow or overflow)
-    if (!INT) *sure = *sure && scale_range(x);
+    if (!INT) *sure = *sure && scale_range(x, c);
     return y;
 }
 
@@ -279,29 +290,27 @@ __device__ __noinline__ float scale_double(float x, float slope, float inter)
 // often (one in 256 with a slope of 0.1, half of them with 0.25 and -3): all of them in FP64
 // took a 224 x 224 x 128 x 4 call to 319 us (8 bits) and 322 us (singles), so 100 and 110.
 template <bool INT>
-__device__ __noinline__ float scale_rest(float x, float slope, float inter)
+__device__ __noinline__ float scale_rest(float x, ScaleF c)
 {
-    const float p = x * slope, pe = fmaf(x, slope, -p), y = fmaf(x, slope, inter);
+    const float slope = c.slope, inter = c.inter, p = x * slope, pe = fmaf(x, slope, -p), y = fmaf(x, slope, inter);
     float te, r1, r2;
     const float t = two_sum(p, inter, &te), s = two_sum(t - y, te, &r1);
     two_sum(s, pe, &r2);
-    if ((INT || scale_range(x)) && r1 == 0.0f && r2 == 0.0f) return y;
+    if ((INT || scale_range(x, c)) && r1 == 0.0f && r2 == 0.0f) return y;
     return scale_double(x, slope, inter);
 }
 
 template <bool INT>
-__device__ __noinline__ float4 scale_quad_rest(float4 e, float slope, float inter)
+__device__ __noinline__ float4 scale_quad_rest(float4 e, ScaleF c)
 {
-    return make_float4(scale_rest<INT>(e.x, slope, inter), scale_rest<INT>(e.y, slope, inter),
-                       scale_rest<INT>(e.z, slope, inter), scale_rest<INT>(e.w, slope, inter));
+    return make_float4(scale_rest<INT>(e.x, c), scale_rest<INT>(e.y, c), scale_rest<INT>(e.z, c), scale_rest<INT>(e.w, c));
 }
 
 constexpr int SCALE_PER = 4;
 
 // scaled 8- and 16-bit and single images whose factors are singles in the middle of the range
 template <typename S, typename O>
-__global__ void __launch_bounds__(256) scale_single_k(O *__restrict__ out, const S *__restrict__ in, Orient o, float slope,
-                                                      float inter)
+__global__ void __launch_bounds__(256) scale_single_k(O *__restrict__ out, const S *__restrict__ in, Orient o, ScaleF c)
 {
     using W = Word<sizeof(S)>;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; r < o.rows; r += (int64_t)gridDim.x * blockDim.y) {
@@ -322,8 +331,8 @@ __global__ void __launch_bounds__(256) scale_single_k(O *__restrict__ out, const
                 S v;
                 memcpy(&v, &w[q], sizeof(S));
                 bool sure;
-                float y = scale_single<(S)0.5 == (S)0>((float)v, slope, inter, &sure);
-                if (!sure) y = scale_rest<(S)0.5 == (S)0>((float)v, slope, inter);
+                float y = scale_single<(S)0.5 == (S)0>((float)v, c, &sure);
+                if (!sure) y = scale_rest<(S)0.5 == (S)0>((float)v, c);
                 if constexpr (sizeof(O) == 8) dst[x] = f32_to_f64(y);
                 else dst[x] = y;
             }
@@ -367,8 +376,7 @@ static QuadWalk quad_walk(const Orient &o)
 }
 
 template <typename S, bool SWAP>
-__global__ void __launch_bounds__(256) scale_quads_k(float *__restrict__ out, const S *__restrict__ in, QuadWalk w, float slope,
-                                                     float inter)
+__global__ void __launch_bounds__(256) scale_quads_k(float *__restrict__ out, const S *__restrict__ in, QuadWalk w, ScaleF f)
 {
     struct alignas(4 * sizeof(S)) Quad {
         typename Word<sizeof(S)>::T w[4];
@@ -397,11 +405,11 @@ __global__ void __launch_bounds__(256) scale_quads_k(float *__restrict__ out, co
             memcpy(&c, &b, sizeof(S));
             e[k] = (float)c;
             bool sure;
-            y[k] = scale_single<(S)0.5 == (S)0>(e[k], slope, inter, &sure);
+            y[k] = scale_single<(S)0.5 == (S)0>(e[k], f, &sure);
             all = all && sure;
         }
         float4 res = make_float4(y[0], y[1], y[2], y[3]);
-        if (!all) res = scale_quad_rest<(S)0.5 == (S)0>(make_float4(e[0], e[1], e[2], e[3]), slope, inter);  // (all four: the same bits)
+        if (!all) res = scale_quad_rest<(S)0.5 == (S)0>(make_float4(e[0], e[1], e[2], e[3]), f);  // (all four: the same bits)
         *reinterpret_cast<float4 *>(out + 4 * (size_t)t) = res;
         q += dq;
         uint32_t c = q >= w.nq;
@@ -773,16 +781,15 @@ qsm_status qsm_nifti_decode(qsm_ctx *ctx, const qsm_nifti_hdr *h, const void *pa
                          o.rows <= 0x7fffffff && (uintptr_t)in % (4 * eb) == 0 && (uintptr_t)so.dev % 16 == 0;
         const unsigned gq = (unsigned)std::min<int64_t>((quads + 255) / 256, 152 * 16);
         const QuadWalk qw = by4 ? quad_walk(o) : QuadWalk{};
+        const ScaleF fac = scale_factors(h->scl_slope, h->scl_inter);
 #define QSM_SCALE(S)                                                                                             \
     if (by4)                                                                                                     \
         (o.swap ? scale_quads_k<S, true> : scale_quads_k<S, false>)<<<gq, 256, 0, ctx->stream>>>(                \
-            (float *)so.dev, (const S *)in, qw, (float)h->scl_slope, (float)h->scl_inter);                       \
+            (float *)so.dev, (const S *)in, qw, fac);                                                            \
     else if (out_datatype == 64)                                                                                      \
-        scale_single_k<S, double><<<g, blk, 0, ctx->stream>>>((double *)so.dev, (const S *)in, o,                \
-                                                              (float)h->scl_slope, (float)h->scl_inter);         \
+        scale_single_k<S, double><<<g, blk, 0, ctx->stream>>>((double *)so.dev, (const S *)in, o, fac);          \
     else                                                                                                         \
-        scale_single_k<S, float><<<g, blk, 0, ctx->stream>>>((float *)so.dev, (const S *)in, o,                  \
-                                                             (float)h->scl_slope, (float)h->scl_inter);
+        scale_single_k<S, float><<<g, blk, 0, ctx->stream>>>((float *)so.dev, (const S *)in, o, fac);
         switch (sdt) {
         case 2: QSM_SCALE(uint8_t) break;
         case 256: QSM_SCALE(int8_t) break;

@@ -192,12 +192,13 @@ def test_scaling_quads(qn, nio, dt, nx, sx, endian):
         assert got.shape == ref.shape and np.array_equal(got, ref)
 
 
-@pytest.mark.parametrize("dt,inter", [(2, -0.3), (16, -3.0)])
-def test_scaling_time_does_not_depend_on_midway_values(qn, dt, inter):
+@pytest.mark.parametrize("dt,inter,unit", [(2, -0.3, 1.0), (16, -3.0, 1.0), (16, 0.0, 1e-14)])
+def test_scaling_time_does_not_depend_on_midway_values(qn, dt, inter, unit):
     """Results midway between two singles are common (8-bit images with a slope of
     0.1: one voxel in 256; singles with 0.25 and -3: half of them) and take about
     the time of an image without any (0.25, and an intercept of 0 for the singles):
-    at most twice, where FP64 per voxel takes over four times."""
+    at most twice, where FP64 per voxel takes over four times.  Nor on the unit of
+    singles (1e-14)."""
     import time
 
     torch = pytest.importorskip("torch")
@@ -205,8 +206,9 @@ def test_scaling_time_does_not_depend_on_midway_values(qn, dt, inter):
     n = 224 * 224 * 128 * 2
     raw = rng.integers(0, 256, n, dtype=np.uint8) if dt == 2 else (rng.standard_normal(n) * 500).astype(np.float32).view(np.uint8)
     dev = torch.from_numpy(raw).cuda()
+    small = dev if dt == 2 else (dev.view(torch.float32) * unit).view(torch.uint8)
 
-    def best(slope, inter):
+    def best(slope, inter, dev=dev):
         hb = build_header("<", datatype=dt, dim=(4, 224, 224, 128, 2, 1, 1, 1), slope=slope, inter=inter)
         ts = []
         for _ in range(20):
@@ -218,7 +220,7 @@ def test_scaling_time_does_not_depend_on_midway_values(qn, dt, inter):
         return min(ts)
 
     plain = best(0.25, -3.0) if dt == 2 else best(0.25, 0.0)
-    ties = best(0.1, inter) if dt == 2 else best(0.25, inter)
+    ties = best(0.1, inter) if dt == 2 else best(0.25, inter, small)
     assert ties < 2 * plain, (ties, plain)
 
 
